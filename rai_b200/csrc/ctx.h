@@ -171,6 +171,8 @@ bool grouped_wants_sorted(int64_t rows, int top, int experts);
 int gemm_tc_pick_splits(rb_ctx* ctx, int64_t m, int64_t n, int64_t k);
 int gemm_reserve_scratch(rb_ctx* ctx, size_t bytes);
 int gemm_simple(rb_ctx* ctx, const GemmArgs& a, int dtype);
+int gemm_f32(rb_ctx* ctx, const GemmArgs& a);   // gemm_f32.cu
+bool gemm_f32_takes(const GemmArgs& a);
 
 // moe.cu: rb_split_append and rb_moe_route, in one launch at single-token steps (route NULL: the first alone)
 struct SplitSpec {

@@ -1,5 +1,5 @@
-// Plain CUDA-core kernels: the float32 data path (rai's F32 models), and a bf16 cross-check of the
-// tensor-core kernels that a developer can select with RAI_B200_SIMPLE=1.  Straightforward
+// Plain CUDA-core kernels: the float32 data path (rai's F32 models; its products are in gemm_f32.cu unless their rows are not made
+// of 16-byte pieces), and a bf16 cross-check of the tensor-core kernels that a developer can select with RAI_B200_SIMPLE=1.  Straightforward
 // shared-memory tiling, float32 accumulation, no tensor cores.
 #include "ctx.h"
 
@@ -67,65 +67,6 @@ __global__ void gemm_plain_kernel(const T* __restrict__ x, const T* __restrict__
     }
 }
 
-// Decode-sized float32 Linear (M <= 8 rows; the reference's examples generate with batch 1 in float32,
-// examples/qwen2/src/main.rs:58).  One warp per output feature: its weight row is read once with 16-byte loads
-// and all M dot products ride along, so the kernel is bound by the weight stream like its bf16 counterpart.
-template <bool GATED>
-__global__ void __launch_bounds__(256) gemv_f32_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                       const float* __restrict__ w2, const float* __restrict__ bias,
-                                                       const float* __restrict__ residual, float* __restrict__ out, int m,
-                                                       int n, int k, int act, const float* __restrict__ act_params, int vec) {
-  const float2 ac = act == RB_ACT_XIELU ? xielu_consts(act_params) : make_float2(0.f, 0.f);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int col = blockIdx.x * 8 + warp;
-  if (col >= n) return;
-  const float* wr = w + (size_t)col * k;
-  const float* wr2 = GATED ? w2 + (size_t)col * k : nullptr;
-  float acc[8], acc2[8];
-#pragma unroll
-  for (int r = 0; r < 8; ++r) { acc[r] = 0.f; acc2[r] = 0.f; }
-  if (vec) {
-    for (int i = lane * 4; i < k; i += 128) {
-      const float4 a = *reinterpret_cast<const float4*>(wr + i);
-      float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (GATED) b = *reinterpret_cast<const float4*>(wr2 + i);
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        if (r >= m) break;
-        const float4 xv = *reinterpret_cast<const float4*>(x + (size_t)r * k + i);
-        acc[r] = fmaf(a.w, xv.w, fmaf(a.z, xv.z, fmaf(a.y, xv.y, fmaf(a.x, xv.x, acc[r]))));
-        if (GATED) acc2[r] = fmaf(b.w, xv.w, fmaf(b.z, xv.z, fmaf(b.y, xv.y, fmaf(b.x, xv.x, acc2[r]))));
-      }
-    }
-  } else {
-    for (int i = lane; i < k; i += 32) {
-      const float a = wr[i], b = GATED ? wr2[i] : 0.f;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        if (r >= m) break;
-        const float xv = x[(size_t)r * k + i];
-        acc[r] = fmaf(a, xv, acc[r]);
-        if (GATED) acc2[r] = fmaf(b, xv, acc2[r]);
-      }
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    if (r >= m) break;
-    float v = warp_sum(acc[r]);
-    const float v2 = GATED ? warp_sum(acc2[r]) : 0.f;
-    if (lane != 0) continue;
-    if (GATED) {
-      v = act_apply(act, v) * v2;
-    } else {
-      if (bias) v += bias[col];
-      v = act_apply(act, v, ac);
-      if (residual) v += residual[(size_t)r * n + col];
-    }
-    out[(size_t)r * n + col] = v;
-  }
-}
-
 // One block per (token, query head): its 8 warps take every 8th key of the paged cache, each with an online
 // softmax of its own (lanes split head_dim), and their (max, sum, O) states are merged through shared memory.
 // float32 throughout.  Correct for any head_dim <= 32 * NJ.
@@ -154,27 +95,55 @@ attention_plain_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, c
   const int first = ext ? first_visible(limit, x.window > 0 ? x.window : 1 << 30, x.chunk) : 0;
   const float slope = ext && x.alibi ? alibi_slope(h, q_heads) : 0.f;
   if (ext) scale *= query_temperature(limit, x.temp_every, x.temp_coef);
-  for (int t = first + warp; t <= limit; t += kPlainAttnWarps) {
-    // sliding window (qwen2.rs:316-334): it acts among the tokens of one call only, the cached prefix stays visible
-    if (!ext && t >= call_base && t + window < limit) continue;
-    const int page = block_table[(size_t)b * pages_per_seq + t / kPageTokens];
-    const size_t off = (((size_t)page * kv_heads + kvh) * kPageTokens + (t % kPageTokens)) * d;
-    float dot = 0.f;
+  // U keys at a time, so that their rows are on the way together and their sums overlap
+  constexpr int U = NJ <= 8 ? 4 : 1;
+  for (int t0 = first + warp; t0 <= limit; t0 += U * kPlainAttnWarps) {
+    T kr[U][NJ], vr[U][NJ];
+    bool seen[U], any = false;
 #pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-      const int i = lane + 32 * j;
-      if (i < d) dot += qv[j] * Cvt<T>::to_f(k_cache[off + i]);
+    for (int u = 0; u < U; ++u) {
+      const int t = t0 + u * kPlainAttnWarps;
+      // sliding window (qwen2.rs:316-334): it acts among the tokens of one call only, the cached prefix stays visible
+      seen[u] = t <= limit && (ext || t < call_base || t + window >= limit);
+      any |= seen[u];
+      if (!seen[u]) continue;
+      const int page = block_table[(size_t)b * pages_per_seq + t / kPageTokens];
+      const size_t off = (((size_t)page * kv_heads + kvh) * kPageTokens + (t % kPageTokens)) * d;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        const int i = lane + 32 * j;
+        if (i < d) { kr[u][j] = k_cache[off + i]; vr[u][j] = v_cache[off + i]; }
+      }
     }
-    dot = warp_sum(dot) * scale;
-    if (ext && x.softcap > 0.f) dot = x.softcap * tanhf(dot / x.softcap);
-    dot = fmaf(-slope, (float)(limit - t), dot);
-    const float mn = fmaxf(mx, dot);
-    const float corr = expf(mx - mn), p = expf(dot - mn);
-    l = l * corr + p;
+    if (!any) continue;
+    float dot[U], mn = mx;
 #pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-      const int i = lane + 32 * j;
-      if (i < d) o[j] = o[j] * corr + p * Cvt<T>::to_f(v_cache[off + i]);
+    for (int u = 0; u < U; ++u) {
+      dot[u] = 0.f;
+      if (!seen[u]) continue;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+        if (lane + 32 * j < d) dot[u] += qv[j] * Cvt<T>::to_f(kr[u][j]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      dot[u] = warp_sum(dot[u]) * scale;
+      if (ext && x.softcap > 0.f) dot[u] = x.softcap * tanhf(dot[u] / x.softcap);
+      dot[u] = fmaf(-slope, (float)(limit - t0 - u * kPlainAttnWarps), dot[u]);
+      if (seen[u]) mn = fmaxf(mn, dot[u]);
+    }
+    const float corr = expf(mx - mn);
+    l *= corr;
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) o[j] *= corr;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (!seen[u]) continue;
+      const float p = expf(dot[u] - mn);
+      l += p;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+        if (lane + 32 * j < d) o[j] += p * Cvt<T>::to_f(vr[u][j]);
     }
     mx = mn;
   }
@@ -271,22 +240,6 @@ attention_talk_plain_kernel(const T* __restrict__ q, const T* __restrict__ k_cac
   }
 }
 
-static bool gemv_f32_launch(rb_ctx* ctx, const GemmArgs& a) {
-  if (a.partials || a.m > 8) return false;
-  auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-  const int vec = (a.k % 4 == 0) && al16(a.x) && al16(a.w) && (!a.w2 || al16(a.w2));
-  const dim3 grid((unsigned)((a.n + 7) / 8));
-  if (a.w2)
-    gemv_f32_kernel<true><<<grid, 256, 0, ctx->stream>>>((const float*)a.x, (const float*)a.w, (const float*)a.w2, nullptr, nullptr,
-                                                         (float*)a.out, (int)a.m, (int)a.n, (int)a.k, a.act, nullptr, vec);
-  else
-    gemv_f32_kernel<false><<<grid, 256, 0, ctx->stream>>>((const float*)a.x, (const float*)a.w, nullptr, (const float*)a.bias,
-                                                          (const float*)a.residual, (float*)a.out, (int)a.m, (int)a.n, (int)a.k,
-                                                          a.act, (const float*)a.act_params, vec);
-  ctx->launches++;
-  return true;
-}
-
 template <typename T>
 static int gemm_plain_launch(rb_ctx* ctx, const GemmArgs& a) {
   const int splits = a.partials ? a.n_split : 1;
@@ -309,7 +262,7 @@ int gemm_simple(rb_ctx* ctx, const GemmArgs& a, int dtype) {
   if (a.m == 0 || a.n == 0) return RB_OK;
   RB_REQUIRE(a.act != RB_ACT_XIELU || (a.act_params && !a.w2), "gemm: RB_ACT_XIELU needs its parameters and an ungated product");
   if (dtype == RB_F32) {
-    if (gemv_f32_launch(ctx, a)) return launch_status("gemv_f32");
+    if (gemm_f32_takes(a)) return gemm_f32(ctx, a);
     return gemm_plain_launch<float>(ctx, a);
   }
   if (dtype == RB_BF16) return gemm_plain_launch<__nv_bfloat16>(ctx, a);

@@ -106,6 +106,7 @@ extern "C" int32_t rb_destroy(rb_ctx* ctx) {
   for (void* r : ctx->retired) cudaFree(r);
   if (ctx->gemm_scratch) cudaFree(ctx->gemm_scratch);
   if (ctx->gemm_tile_count) cudaFree(ctx->gemm_tile_count);
+  for (PairSpace& p : ctx->pair_space) { cudaFree(p.slabs); cudaFree(p.flags); }
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
   delete ctx;
   return RB_OK;
@@ -138,6 +139,8 @@ extern "C" int32_t rb_sync(rb_ctx* ctx) {
       RB_CUDA(cudaMemset(ctx->argmax_best, 0, kArgmaxRows * sizeof(unsigned long long)));
       RB_CUDA(cudaMemset(ctx->argmax_count, 0, kArgmaxRows * sizeof(unsigned int)));
       RB_CUDA(cudaMemset(ctx->gemm_tile_count, 0, 2 * kGemmMaxReduceTiles * sizeof(uint32_t)));
+      for (PairSpace& p : ctx->pair_space)
+        if (p.flags) RB_CUDA(cudaMemset(p.flags, 0, kPairFlagBytes));
     }
     return fail(code, "device-side check failed: code %d at 0x%x (detail %u, %u)", code, w[1], w[2], w[3]);
   }

@@ -9,6 +9,17 @@
 
 #include "common.cuh"
 
+// What clusters that share a GEMM tile leave for one another (gemm_pair.cu): float32 sums and flags that the reader clears.
+// One per stream, for the first kPairStreams streams that need one.
+constexpr int kPairStreams = 4, kPairClusters = 74;
+constexpr size_t kPairSlabBytes = (size_t)kPairClusters * 4 * 128 * 256 * sizeof(float);
+constexpr size_t kPairFlagBytes = (size_t)kPairClusters * 4 * 8 * sizeof(uint32_t);
+struct PairSpace {
+  cudaStream_t stream = nullptr;
+  float* slabs = nullptr;
+  uint32_t* flags = nullptr;
+};
+
 struct rb_ctx {
   int device = 0;
   cudaStream_t own_stream = nullptr;
@@ -26,6 +37,7 @@ struct rb_ctx {
   float* gemm_scratch = nullptr;   // float32 slabs of the GEMMs that reduce split-K inside the kernel; grow-only
   size_t gemm_scratch_bytes = 0;
   uint32_t* gemm_tile_count = nullptr;  // [2][kGemmMaxReduceTiles] arrival / done counters of those GEMMs, self-resetting
+  PairSpace pair_space[kPairStreams];
   long long wait_budget_cycles = 2000000000LL;  // give-up time of a device-side wait for ANOTHER GPU (rb_set_wait_budget_us)
   // Waits inside one kernel (operand rings, accumulators, sibling blocks) may begin before the kernel's predecessor
   // has finished, and that predecessor may itself be waiting for a peer: they get four times the budget, so that
@@ -165,6 +177,7 @@ struct GemmArgs {
   bool reduce = false;            // M <= 64: if K is split, sum the splits inside the kernel and apply the epilogue
 };
 int gemm_tc_bf16(rb_ctx* ctx, const GemmArgs& a);
+int gemm_pair_bf16(rb_ctx* ctx, const GemmArgs& a);   // gemm_pair.cu: M > 256, no partials
 constexpr int kMaxExperts = 256;
 int gemm_tc_grouped(rb_ctx* ctx, const GemmArgs& a);
 bool grouped_wants_sorted(int64_t rows, int top, int experts);

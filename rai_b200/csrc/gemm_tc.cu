@@ -13,7 +13,7 @@
 //
 // Operands are named by the TMEM axis they feed: the P operand's rows become TMEM lanes (128 per
 // tile), the Q operand's rows become TMEM columns (BN per tile).
-//   normal (SWAP = false): P = X, Q = W  — prefill-sized M.
+//   normal (SWAP = false): P = X, Q = W  — experts with many rows each (plain prefill-sized products: gemm_pair.cu).
 //   swapped (SWAP = true):  P = W, Q = X  — decode-sized M (<= 256): the weight matrix, which is
 //            all of the HBM traffic, streams through the 128-row side at full tile efficiency while
 //            the few activation rows ride along as the narrow N side.  Two forms of split-K, both through
@@ -46,6 +46,7 @@
 #include <vector>
 
 #include "ctx.h"
+#include "gemm_epilogue.cuh"
 #include "groups.cuh"
 #include "ptx.cuh"
 
@@ -109,23 +110,11 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
   return v;
 }
 
-__device__ __forceinline__ void decode_item(const Params& p, int item, bool swap, int& pt, int& qt, int& split) {
-  if (swap) {
-    split = item % p.n_split;
-    const int tile = item / p.n_split;
-    qt = tile % p.n_q;
-    pt = tile / p.n_q;
-  } else {
-    split = 0;
-    constexpr int G = 16;  // P tiles per raster group: concurrent CTAs share operand tiles in L2
-    const int per_group = G * p.n_q;
-    const int group = item / per_group;
-    const int first = group * G;
-    const int gsz = min(p.n_p - first, G);
-    const int in_group = item % per_group;
-    pt = first + in_group % gsz;
-    qt = in_group / gsz;
-  }
+__device__ __forceinline__ void decode_item(const Params& p, int item, int& pt, int& qt, int& split) {
+  split = item % p.n_split;
+  const int tile = item / p.n_split;
+  qt = tile % p.n_q;
+  pt = tile / p.n_q;
 }
 
 // GROUP: the expert, weight tile and row tile (of `tile` rows) of an item; neighbouring items share a weight tile
@@ -136,75 +125,16 @@ __device__ __forceinline__ void group_item(const Groups& g, int E, int item, int
   rt = at % n_rt;
 }
 
-__device__ __forceinline__ uint4 pack8(const float* v) {
-  uint4 r;
-  __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]);
-  __nv_bfloat162 b = __floats2bfloat162_rn(v[2], v[3]);
-  __nv_bfloat162 c = __floats2bfloat162_rn(v[4], v[5]);
-  __nv_bfloat162 d = __floats2bfloat162_rn(v[6], v[7]);
-  r.x = *reinterpret_cast<uint32_t*>(&a);
-  r.y = *reinterpret_cast<uint32_t*>(&b);
-  r.z = *reinterpret_cast<uint32_t*>(&c);
-  r.w = *reinterpret_cast<uint32_t*>(&d);
-  return r;
-}
-__device__ __forceinline__ void unpack8(const uint4& u, float* v) {
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 f = __bfloat1622float2(h[i]);
-    v[2 * i] = f.x;
-    v[2 * i + 1] = f.y;
-  }
-}
-
 constexpr int kEpiPitch = kBM + 8;  // elements; keeps the 16-byte row reads of the staging tile conflict-free
 
 // Barrier among the 128 epilogue threads only (hardware barrier 1; __syncthreads is barrier 0).
 __device__ __forceinline__ void epi_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
-__device__ __forceinline__ float tanh_fast(float x) {
-  float y;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// Activation over a register array with the selector hoisted out of the element loop
-// (rai-core/src/hlops/activations.rs:20-32); fast-math forms, results are rounded to bf16 anyway.
-template <int N>
-__device__ __forceinline__ void act_inplace(int act, float (&v)[N], float2 ac) {
-  if (act == RB_ACT_SILU) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) v[i] = __fdividef(v[i], 1.0f + __expf(-v[i]));
-  } else if (act == RB_ACT_GELU_TANH) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      const float x = v[i];
-      v[i] = 0.5f * x * (1.0f + tanh_fast(0.7978845608028654f * (x + 0.044715f * x * x * x)));
-    }
-  } else if (act == RB_ACT_GELU_ERF) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) v[i] = v[i] * 0.5f * (1.0f + erff(v[i] * 0.7071067811865476f));
-  } else if (act == RB_ACT_RELU) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) v[i] = fmaxf(v[i], 0.f);
-  } else if (act == RB_ACT_RELU2) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) { const float r = fmaxf(v[i], 0.f); v[i] = r * r; }
-  } else if (act == RB_ACT_XIELU) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      const float z = v[i];
-      const float curve = z > 0.f ? ac.x * z * z : ac.y * (__expf(fminf(z, 0.f)) - 1.0f - z);
-      v[i] = fmaf(0.5f, z, curve);
-    }
-  }
-}
-
 template <int BN, bool SWAP, bool GATED, int GROUP>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__ CUtensorMap tm_p2,
                const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_q2, const Params p) {
+  static_assert(SWAP || GROUP != 0, "plain products of many rows: gemm_pair.cu");
   constexpr bool kGather = GROUP != 0 && SWAP;  // rows by index
   static_assert(!kGather || BN <= 128, "one gather per lane");
   constexpr int kRowTile = SWAP ? BN : kBM;
@@ -314,29 +244,22 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
       // decode-sized GEMMs read every weight byte exactly once: evict-first keeps them from pushing
       // the activations and split-K partials out of L2
       const uint64_t stream_policy = ptx::policy_evict_first();
-      auto load_weights = [&](uint8_t* st, int stage, int kb, int pt, int qt) {
-        if (SWAP) {
-          ptx::tma_load_2d_hint(st, &tm_p, &full_bar[stage], kb * kBK, pt * kBM, stream_policy);
-          if (C::kPTiles == 2)
-            ptx::tma_load_2d_hint(st + C::kPBytes, &tm_p2, &full_bar[stage], kb * kBK, pt * kBM, stream_policy);
-        } else {
-          uint8_t* qs = st + C::kPTiles * C::kPBytes;
-          ptx::tma_load_2d(qs, &tm_q, &full_bar[stage], kb * kBK, qt * BN);
-          if (C::kQTiles == 2) ptx::tma_load_2d(qs + C::kQBytes, &tm_q2, &full_bar[stage], kb * kBK, qt * BN);
-        }
+      auto load_weights = [&](uint8_t* st, int stage, int kb, int pt) {
+        ptx::tma_load_2d_hint(st, &tm_p, &full_bar[stage], kb * kBK, pt * kBM, stream_policy);
+        if (C::kPTiles == 2)
+          ptx::tma_load_2d_hint(st + C::kPBytes, &tm_p2, &full_bar[stage], kb * kBK, pt * kBM, stream_policy);
       };
-      auto load_activations = [&](uint8_t* st, int stage, int kb, int pt, int qt) {
-        if (SWAP) ptx::tma_load_2d(st + C::kPTiles * C::kPBytes, &tm_q, &full_bar[stage], kb * kBK, qt * BN);
-        else ptx::tma_load_2d(st, &tm_p, &full_bar[stage], kb * kBK, pt * kBM);
+      auto load_activations = [&](uint8_t* st, int stage, int kb, int qt) {
+        ptx::tma_load_2d(st + C::kPTiles * C::kPBytes, &tm_q, &full_bar[stage], kb * kBK, qt * BN);
       };
       int n_pre = 0;
       for (int item = blockIdx.x; item < p.n_items && n_pre < n_stages; item += gridDim.x) {
         int pt, qt, split;
-        decode_item(p, item, SWAP, pt, qt, split);
+        decode_item(p, item, pt, qt, split);
         const int kb0 = split * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
         for (int kb = kb0; kb < kb1 && n_pre < n_stages; ++kb, ++n_pre) {
           ptx::mbar_expect_tx(&full_bar[n_pre], C::kStageBytes);
-          load_weights(tiles + (size_t)n_pre * C::kStageBytes, n_pre, kb, pt, qt);
+          load_weights(tiles + (size_t)n_pre * C::kStageBytes, n_pre, kb, pt);
         }
       }
       pdl_wait();
@@ -346,16 +269,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
       bool ok = true;
       for (int item = blockIdx.x; item < p.n_items && ok; item += gridDim.x) {
         int pt, qt, split;
-        decode_item(p, item, SWAP, pt, qt, split);
+        decode_item(p, item, pt, qt, split);
         const int kb0 = split * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
         for (int kb = kb0; kb < kb1; ++kb) {
           uint8_t* st = tiles + (size_t)stage * C::kStageBytes;
           if ((int)issued >= n_pre) {
             if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1u, &abort_flag, p.wait_cycles)) { ok = false; break; }
             ptx::mbar_expect_tx(&full_bar[stage], C::kStageBytes);
-            load_weights(st, stage, kb, pt, qt);
+            load_weights(st, stage, kb, pt);
           }
-          load_activations(st, stage, kb, pt, qt);
+          load_activations(st, stage, kb, qt);
           ++issued;
           if (++stage == n_stages) { stage = 0; phase ^= 1u; }
         }
@@ -366,7 +289,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (lane == 0) {
-      constexpr uint32_t idesc = ptx::umma_idesc_bf16(kBM, BN);
+      // gate and up rows of a stage lie one below the other: one product covers both, and reads X once
+      constexpr bool kBoth = GATED && !SWAP;
+      constexpr uint32_t idesc = ptx::umma_idesc_bf16(kBM, kBoth ? 2 * BN : BN);
       int stage = 0;
       uint32_t phase = 0;
       int as = 0;
@@ -374,7 +299,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
       bool ok = true;
       for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
         int pt, qt, split = 0;
-        if (GROUP == 0) decode_item(p, item, SWAP, pt, qt, split);
+        if (GROUP == 0) decode_item(p, item, pt, qt, split);
         const int kb0 = split * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
         if (kb0 >= kb1) continue;  // empty split: the epilogue writes zeros on its own
         if (!ptx::mbar_wait(&acc_empty[as], aphase ^ 1u, &abort_flag, p.wait_cycles)) { ok = false; break; }
@@ -390,7 +315,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
           for (int j = 0; j < kBK / 16; ++j) {
             const uint32_t acc = (kb > kb0 || j > 0) ? 1u : 0u;
             ptx::umma_bf16(d0, ptx::umma_desc_k_sw128(p0 + j * 32), ptx::umma_desc_k_sw128(q0 + j * 32), idesc, acc);
-            if (GATED)
+            if (GATED && !kBoth)
               ptx::umma_bf16(d0 + BN, ptx::umma_desc_k_sw128(p1 + j * 32), ptx::umma_desc_k_sw128(q1 + j * 32), idesc,
                              acc);
           }
@@ -425,7 +350,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
         m_lim = groups.row[e + 1] - row0;
         if (GROUP == 2) scatter = p.list + (size_t)e * p.cap;
       } else {
-        decode_item(p, item, SWAP, pt, qt, split);
+        decode_item(p, item, pt, qt, split);
       }
       if (split * p.kb_per_split >= p.num_kb) {  // empty split (only with partials): zero slab, no accumulator
         const int gn = pt * kBM + lane_row;
@@ -538,9 +463,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
           const int gm = pt * kBM + lane_row;
           const int gn0 = qt * BN + c0;
           if (GATED) act_inplace(p.act, g, ac);
+          else if (p.act != RB_ACT_NONE) act_inplace(p.act, v, ac);
           if (gm < m_lim) {
-            const bool vec_ok = (p.n % 8) == 0;
-            const size_t o_row = GROUP == 0 ? gm : GROUP == 1 ? row0 + gm : scatter[gm];
+            const size_t o_row = GROUP == 1 ? row0 + gm : scatter[gm];  // (their columns come in eights)
 #pragma unroll
             for (int j8 = 0; j8 < CH; j8 += 8) {
               const int gn = gn0 + j8;
@@ -552,34 +477,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
               } else {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) y[j] = v[j8 + j];
-                if (p.bias) {
-                  if (vec_ok) {
-                    float b8[8];
-                    unpack8(*reinterpret_cast<const uint4*>(p.bias + gn), b8);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) y[j] += b8[j];
-                  } else {
-                    for (int j = 0; j < 8 && gn + j < p.n; ++j) y[j] += __bfloat162float(p.bias[gn + j]);
-                  }
-                }
-                act_inplace(p.act, y, ac);
-                if (p.residual) {
-                  if (vec_ok) {
-                    float r8[8];
-                    unpack8(*reinterpret_cast<const uint4*>(p.residual + (size_t)gm * p.n + gn), r8);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) y[j] += r8[j];
-                  } else {
-                    for (int j = 0; j < 8 && gn + j < p.n; ++j)
-                      y[j] += __bfloat162float(p.residual[(size_t)gm * p.n + gn + j]);
-                  }
-                }
               }
-              if (vec_ok) {
-                *reinterpret_cast<uint4*>(p.out + o_row * p.n + gn) = pack8(y);
-              } else {
-                for (int j = 0; j < 8 && gn + j < p.n; ++j) p.out[(size_t)gm * p.n + gn + j] = __float2bfloat16_rn(y[j]);
-              }
+              *reinterpret_cast<uint4*>(p.out + o_row * p.n + gn) = pack8(y);
             }
           }
         }
@@ -599,7 +498,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
       // epilogue to that slice.  The last one to finish reading re-arms the tile's counters for the next launch.
       const int et = threadIdx.x - 64;
       int pt, qt, split;
-      decode_item(p, blockIdx.x, true, pt, qt, split);
+      decode_item(p, blockIdx.x, pt, qt, split);
       const int tile = pt * p.n_q + qt;
       const int ns = p.n_split;
       epi_barrier();  // the epilogue threads' slab stores precede thread 0's fence
@@ -896,9 +795,7 @@ int gemm_tc_bf16(rb_ctx* ctx, const GemmArgs& a) {
     if (a.m <= 128) return launch<128, true, false>(ctx, a, p);
     return launch<256, true, false>(ctx, a, p);
   }
-  p.p_rows = (int)a.m; p.q_rows = (int)a.n;
-  if (gated) return launch<128, false, true>(ctx, a, p);
-  return launch<256, false, false>(ctx, a, p);
+  return gemm_pair_bf16(ctx, a);
 }
 
 // The grouped form: a.m is the number of (row, choice) pairs.  a.x has a.m / a.top rows (a.up), or a.m compact rows (down, or

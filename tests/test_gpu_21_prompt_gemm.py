@@ -1,4 +1,5 @@
-"""The float32 products at the edges of their tiles, against float64 sums of the same operands."""
+"""The products of prompts: the paired-SM bf16 kernel at the edges of its tiles and with tiles cut along K, and the float32
+kernels at the edges of theirs, against float32 / float64 sums of the same operands."""
 import ctypes
 
 import pytest
@@ -33,6 +34,70 @@ def linear_ref(x, w, b, r, act):
     y = y + b.double() if b is not None else y
     y = torch.nn.functional.silu(y) if act == _lib.ACT_SILU else y
     return y + r.double() if r is not None else y
+
+
+# one row more or less than a tile of 256 or 512; columns that end in a tile, in a piece of eight and (250) within one; K of part
+# of a slice; few tiles with many slices (cut among all clusters), and a little more than one tile for each cluster
+SHAPES = [(257, 256, 64), (511, 264, 72), (512, 8, 8), (513, 250, 192), (300, 512, 8192), (1300, 4096, 2048), (770, 2816, 6400),
+          (4096, 2560, 1024), (2600, 1000, 328)]
+
+
+@pytest.mark.parametrize("m,n,k", SHAPES)
+def test_prompt_products(cuda, m, n, k):
+    cuda.use_torch_stream()
+    x, w, w2, b, r = operands(m, n, k, torch.bfloat16, m + n + k)
+    for bias, res, act in ((None, None, _lib.ACT_NONE), (b, r, _lib.ACT_SILU)):
+        out = linear(cuda, x, w, bias, res, act)
+        cuda.synchronize()
+        ref = linear_ref(x, w, bias, res, act)
+        assert float((out.double() - ref).abs().max()) <= bound(torch.bfloat16, ref, k)
+    # the residual may be the output itself, and a second pass over fresh sums gives the same bits
+    again, once = r.clone(), linear(cuda, x, w, None, r, _lib.ACT_NONE)
+    _lib.call("rb_linear", cuda.ctx, P(x), P(w), None, P(again), P(again), m, n, k, _lib.ACT_NONE, _lib.BF16)
+    cuda.synchronize()
+    assert torch.equal(again, once)
+    if n % 8 == 0:
+        out = torch.full((m, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+        _lib.call("rb_gated_linear", cuda.ctx, P(x), P(w), P(w2), P(out), m, n, k, _lib.ACT_SILU, _lib.BF16)
+        cuda.synchronize()
+        ref = torch.nn.functional.silu(x.double() @ w.double().t()) * (x.double() @ w2.double().t())
+        assert float((out.double() - ref).abs().max()) <= 2 * bound(torch.bfloat16, ref, k)  # (and a fast exponential)
+
+
+def test_infinities_and_nan_stay_in_their_rows(cuda):
+    cuda.use_torch_stream()
+    x, w, _, _, _ = operands(600, 512, 4096, torch.bfloat16, 7)
+    clean = linear(cuda, x, w, None, None, _lib.ACT_NONE)
+    x2 = x.clone()
+    x2[599, 5], x2[300, 4000] = float("nan"), float("inf")
+    out = linear(cuda, x2, w, None, None, _lib.ACT_NONE)
+    cuda.synchronize()
+    assert torch.isnan(out[599]).all() and not torch.isfinite(out[300]).any()
+    keep = [i for i in range(600) if i not in (300, 599)]
+    assert torch.equal(out[keep], clean[keep])
+
+
+def test_cut_tiles_on_several_streams_and_under_capture(cuda):
+    """Streams have workspaces of their own; a captured launch, and a stream too many, use whole tiles."""
+    x, w, _, _, _ = operands(300, 512, 8192, torch.bfloat16, 3)
+    ref = linear_ref(x, w, None, None, _lib.ACT_NONE)
+    streams, outs = [torch.cuda.Stream() for _ in range(2)], []
+    torch.cuda.synchronize()
+    for s in streams * 3 + [torch.cuda.Stream() for _ in range(6)]:
+        with torch.cuda.stream(s):
+            cuda.use_torch_stream()
+            outs.append(linear(cuda, x, w, None, None, _lib.ACT_NONE))
+    torch.cuda.synchronize()
+    graph, static = torch.cuda.CUDAGraph(), torch.zeros(300, 512, dtype=torch.bfloat16, device="cuda")
+    with torch.cuda.graph(graph):
+        cuda.use_torch_stream()
+        _lib.call("rb_linear", cuda.ctx, P(x), P(w), None, None, P(static), 300, 512, 8192, _lib.ACT_NONE, _lib.BF16)
+    graph.replay()
+    torch.cuda.synchronize()
+    cuda.use_torch_stream()
+    cuda.synchronize()
+    for out in outs + [static]:
+        assert float((out.double() - ref).abs().max()) <= bound(torch.bfloat16, ref, 8192)
 
 
 # rows: few (a dot product per row) and many (tiles of 16 to 128 rows); features around a tile; K cut in up to eight shares, not a

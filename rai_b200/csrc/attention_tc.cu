@@ -1,4 +1,4 @@
-// Causal prefill attention on the 5th-generation tensor cores, for head sizes 64 and 128 and query lengths of at
+// Causal prefill attention on the 5th-generation tensor cores, for head sizes 64, 80, 96, 128 and 256 and query lengths of at
 // least one tile: softmax(Q K^T * scale + mask) V over the paged bf16 KV cache without materialising scores
 // (rai-models/src/llm/qwen2.rs:205-216 and its phi3 / gemma twins; the fused op the reference itself has for this
 // is ops::FlashAttention, rai-core/src/ops/flash_attention.rs:154-176).
@@ -19,6 +19,9 @@
 // The score MMA of tile j+1 is issued before the P.V MMA of tile j, so the tensor pipe computes the next scores while
 // the softmax warps work on the current ones; two CTAs fit per SM (112 KB of shared memory, 256 TMEM columns
 // each), which overlaps one CTA's softmax with the other's MMAs.
+// Operand tiles come in column blocks of 64.  The second block of heads of 80 and 96 is partly empty: zeros in K and V (beyond
+// their rows' end), the next head's columns in Q; the products take head_dim columns and never read it.  Heads of 256 take
+// 208 KB of shared memory and 384 TMEM columns, so one CTA per SM.
 // Where the values are the keys (EXT == 2) a tile is loaded once, serves both products from a ring of four, and is released
 // after P.V.
 //
@@ -46,15 +49,16 @@ template <int D, bool SHARED = false>
 struct TCfg {
   // the values are the keys: one ring over the space of both, a tile is released once both products have read it
   static constexpr int kRing = SHARED ? 4 : 2;
-  static constexpr int kQBytes = kBM * D * 2;   // [D/64 column blocks][128 rows][128 bytes]
-  static constexpr int kKBytes = kBN * D * 2;   // [D/64][64 keys][128 bytes]
-  static constexpr int kVBytes = kBN * D * 2;
+  static constexpr int kBlocks = (D + 63) / 64;
+  static constexpr int kQBytes = kBM * kBlocks * 128;   // [column blocks of 64][128 rows][128 bytes]
+  static constexpr int kKBytes = kBN * kBlocks * 128;   // [column blocks][64 keys][128 bytes]
+  static constexpr int kVBytes = kKBytes;
   static constexpr int kPBytes = kBM * kBN * 2;  // [128 rows][128 bytes]
   static constexpr int kTileBytes = kQBytes + 2 * kKBytes + 2 * kVBytes + kPBytes;
   static constexpr int kBarBytes = 256;          // barriers and control words, after the tiles
   // at least 100 KB, so that never more than two CTAs (256 TMEM columns each) share an SM
   static constexpr int kSmemBytes = (kTileBytes + kBarBytes) > 100 * 1024 ? (kTileBytes + kBarBytes) : 100 * 1024;
-  static constexpr int kTmemCols = 256;          // two score buffers of 64 columns, then O (head_dim columns)
+  static constexpr int kTmemCols = D <= 128 ? 256 : 512;  // two score buffers of 64 columns, then O (head_dim columns)
   static constexpr uint32_t kOCol = 2 * kBN;
 };
 
@@ -121,7 +125,7 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 
 // EXT: 0 = plain causal, 1 = with what AttnExtra names, 2 = that over a cache whose values are its keys
 template <int D, int EXT>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, D <= 128 ? 2 : 1)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                             const __grid_constant__ CUtensorMap tm_v, const TParams p) {
   constexpr bool SHARED = EXT == 2;
@@ -182,7 +186,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
     if (lane == 0) {
       ptx::mbar_expect_tx(&ctl->q_full, C::kQBytes);
 #pragma unroll
-      for (int cb = 0; cb < D / 64; ++cb)
+      for (int cb = 0; cb < C::kBlocks; ++cb)
         ptx::tma_load_2d(q_s + cb * (kBM * 128), &tm_q, &ctl->q_full, head * D + cb * 64, b * p.s_new + q0);
       bool ok = true;
       for (int j = 0; j < n && ok; ++j) {
@@ -193,14 +197,14 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
         if (!ptx::mbar_wait(&ctl->k_empty[kst], kph ^ 1u, abort_flag, p.wait_cycles)) { ok = false; break; }
         ptx::mbar_expect_tx(&ctl->k_full[kst], C::kKBytes);
 #pragma unroll
-        for (int cb = 0; cb < D / 64; ++cb)
+        for (int cb = 0; cb < C::kBlocks; ++cb)
           ptx::tma_load_2d(k_s + kst * C::kKBytes + cb * (kBN * 128), &tm_k, &ctl->k_full[kst], cb * 64, y);
         ctl->k_issued = (uint32_t)(j + 1);
         if (SHARED) continue;
         if (!ptx::mbar_wait(&ctl->v_empty[st], ph ^ 1u, abort_flag, p.wait_cycles)) { ok = false; break; }
         ptx::mbar_expect_tx(&ctl->v_full[st], C::kVBytes);
 #pragma unroll
-        for (int cb = 0; cb < D / 64; ++cb)
+        for (int cb = 0; cb < C::kBlocks; ++cb)
           ptx::tma_load_2d(v_s + st * C::kVBytes + cb * (kBN * 128), &tm_v, &ctl->v_full[st], cb * 64, y);
         ctl->v_issued = (uint32_t)(j + 1);
       }
@@ -465,6 +469,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
         } else if (store) {
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {
+            if (D % 32 != 0 && c0 + i >= D) break;
             float v[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) v[k] = __uint_as_float(r[i + k]) * inv;
@@ -574,10 +579,11 @@ int launch_tc(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, 
 
 }  // namespace
 
-bool attention_prefill_tc_supported(const rb_kv_cache* c, int s_new, int q_heads, const void* q, const void* out) {
+bool attention_prefill_tc_supported(const rb_kv_cache* c, int s_new, int q_heads, const void* q, const void* out, bool extra) {
   auto al16 = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; };
-  return c->dtype == RB_BF16 && (c->head_dim == 64 || c->head_dim == 128) && s_new >= kBM && q_heads % c->kv_heads == 0 &&
-         al16(q) && al16(out);
+  const int d = c->head_dim;
+  return c->dtype == RB_BF16 && (d == 64 || d == 128 || (!extra && (d == 80 || d == 96 || d == 256))) && s_new >= kBM &&
+         q_heads % c->kv_heads == 0 && al16(q) && al16(out);
 }
 
 int attention_prefill_tc(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, int s_new, int q_heads, float scale,
@@ -588,7 +594,10 @@ int attention_prefill_tc(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, 
   };
   if (c->head_dim == 64) return go(launch_tc<64, 0>, launch_tc<64, 1>, launch_tc<64, 2>);
   if (c->head_dim == 128) return go(launch_tc<128, 0>, launch_tc<128, 1>, launch_tc<128, 2>);
-  return fail(RB_ERR_UNIMPLEMENTED, "tensor-core prefill attention: head_dim %d unsupported (64, 128)", c->head_dim);
+  if (kind == 0 && c->head_dim == 80) return launch_tc<80, 0>(ctx, q, c, layer, batch, s_new, q_heads, scale, out, ext);
+  if (kind == 0 && c->head_dim == 96) return launch_tc<96, 0>(ctx, q, c, layer, batch, s_new, q_heads, scale, out, ext);
+  if (kind == 0 && c->head_dim == 256) return launch_tc<256, 0>(ctx, q, c, layer, batch, s_new, q_heads, scale, out, ext);
+  return fail(RB_ERR_UNIMPLEMENTED, "tensor-core prefill attention: head_dim %d unsupported", c->head_dim);
 }
 
 }  // namespace rb

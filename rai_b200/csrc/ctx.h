@@ -319,8 +319,8 @@ inline int attention_walk_len(int max_len, int window, int chunk = 0) {
   return (window > 0 && window < max_len - 64) ? window + 64 : max_len;
 }
 int attention_reserve_scratch(rb_ctx* ctx, size_t bytes);
-// attention_tc.cu: causal prefill attention on tcgen05 (head sizes 64 and 128, query length >= 128)
-bool attention_prefill_tc_supported(const rb_kv_cache* c, int s_new, int q_heads, const void* q, const void* out);
+// attention_tc.cu: causal prefill attention on tcgen05 (head sizes 64 and 128, without `extra` also 80, 96 and 256; query length >= 128)
+bool attention_prefill_tc_supported(const rb_kv_cache* c, int s_new, int q_heads, const void* q, const void* out, bool extra);
 int attention_prefill_tc(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, int s_new, int q_heads, float scale,
                          void* out, const AttnExtra* ext = nullptr);
 // attention_latent.cu, attention_talk.cu: attention with mixed heads or over latents, one block for all heads of its tokens

@@ -491,26 +491,33 @@ extern "C" int32_t rb_rope_attention_decode(rb_ctx* ctx, const void* qkv, const 
 
 extern "C" int32_t rb_attention(rb_ctx* ctx, const void* q, rb_kv_cache* c, int32_t layer, int32_t batch, int32_t s_new,
                                 int32_t q_heads, float scale, void* out, int32_t dtype) {
+  return attention_rows(ctx, q, c, layer, batch, s_new, q_heads, scale, out, dtype, nullptr);
+}
+
+int rb::attention_rows(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, int s_new, int q_heads, float scale, void* out,
+                       int dtype, const Packed* pk) {
   RB_REQUIRE(ctx && q && c && out, "rb_attention: null argument");
   RB_REQUIRE(dtype == c->dtype, "rb_attention: cache dtype differs");
   RB_REQUIRE(layer >= 0 && layer < c->layers, "rb_attention: layer %d out of range", layer);
   RB_REQUIRE(batch > 0 && batch <= c->max_batch && s_new > 0, "rb_attention: bad batch/seq");
   RB_REQUIRE(q_heads > 0 && q_heads % c->kv_heads == 0, "rb_attention: %d query heads over %d KV heads", q_heads,
              c->kv_heads);
-  for (int b = 0; b < batch; ++b)
+  for (int b = 0; !pk && b < batch; ++b)
     RB_REQUIRE(c->host_lens[b] >= s_new, "rb_attention: sequence %d holds %d tokens, fewer than the %d new ones", b,
                c->host_lens[b], s_new);
   double kv_tokens = 0.0, pairs = 0.0;  // keys read; (query, key) pairs under the causal mask
   for (int b = 0; b < batch; ++b) {
     const double len = c->host_lens[b];
     kv_tokens += len;
-    pairs += (double)s_new * (len - s_new) + 0.5 * s_new * (s_new + 1.0);
+    const double fresh = pk ? (double)pk->rows / batch : s_new;  // (packed: the mean)
+    pairs += fresh * (len - fresh) + 0.5 * fresh * (fresh + 1.0);
   }
   const double es = (double)dtype_size(dtype), d = c->head_dim;
   ProfScope prof(ctx, RB_PROF_ATTENTION,
-                 es * (2.0 * kv_tokens * c->kv_heads * d + 2.0 * batch * s_new * q_heads * d), 4.0 * pairs * q_heads * d);
-  if (dtype == RB_BF16 && !ctx->debug_simple_attn) return attention_mma_bf16(ctx, q, c, layer, batch, s_new, q_heads, scale, out);
-  return attention_simple(ctx, q, c, layer, batch, s_new, q_heads, scale, out, dtype);
+                 es * (2.0 * kv_tokens * c->kv_heads * d + 2.0 * (pk ? pk->rows : batch * s_new) * q_heads * d), 4.0 * pairs * q_heads * d);
+  if (dtype == RB_BF16 && !ctx->debug_simple_attn) 
+    return attention_mma_bf16(ctx, q, c, layer, batch, s_new, q_heads, scale, out, nullptr, pk);
+  return attention_simple(ctx, q, c, layer, batch, s_new, q_heads, scale, out, dtype, nullptr, pk);
 }
 
 extern "C" int32_t rb_attention_window(rb_ctx* ctx, const void* q, rb_kv_cache* c, int32_t layer, int32_t batch, int32_t s_new,

@@ -102,6 +102,7 @@ struct AParams {
   const int32_t* block_table;
   const int32_t* seq_lens;
   int pages_per_seq, s_new, q_heads, kv_heads, group;
+  const int32_t* start = nullptr;  // prompts: Packed::start, or NULL
   int n_splits;
   int window;      // sliding window (qwen2.rs:316-327): among the tokens of one call, key j is hidden from row i when j + window < i
   long long wait_cycles;  // give-up budget of the bounded waits
@@ -187,7 +188,10 @@ attention_kernel(const AParams p, const __grid_constant__ CUtensorMap tm_k, cons
   }
   // (fused step: read before the dependency wait, so straight from L2, where the kernel that set it left it)
   const int len = fuse ? __ldcg(p.seq_lens + b) : p.seq_lens[b];
-  const int base = len - p.s_new;  // absolute position of query row 0
+  const int s_new = DECODE ? 1 : rows_of(p.start, b, p.s_new);
+  if (!DECODE && q0 >= s_new) return;  // a ragged batch: the grid is made for its longest sequence
+  const int q_row = DECODE ? b : first_row(p.start, b, p.s_new) + q0;  // of q and out
+  const int base = len - s_new;  // absolute position of query row 0
 
   // key tiles this CTA walks
   int tile_lo, tile_hi;
@@ -337,7 +341,7 @@ attention_kernel(const AParams p, const __grid_constant__ CUtensorMap tm_k, cons
       if (DECODE) {
         if (r < p.group) src = p.q + ((size_t)b * p.q_heads + head + r) * D + c * 8;
       } else {
-        if (q0 + r < p.s_new) src = p.q + (((size_t)b * p.s_new + q0 + r) * p.q_heads + head) * D + c * 8;
+        if (q0 + r < s_new) src = p.q + ((size_t)(q_row + r) * p.q_heads + head) * D + c * 8;
       }
       const uint32_t dst = s_u32(q_s + r * C::kRowBytes + c * 16);
       if (src) cp_async16(dst, src);
@@ -523,8 +527,8 @@ attention_kernel(const AParams p, const __grid_constant__ CUtensorMap tm_k, cons
   if (!DECODE) {
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) {
-      const int row = q0 + qrow0 + g + hf * 8;
-      if (row >= p.s_new) continue;
+      const int r = qrow0 + g + hf * 8;
+      if (q0 + r >= s_new) continue;
       if (EXT && p.x_sink) l_run[hf] += exp2f(__bfloat162float(p.x_sink[head]) * kLog2e - m_run[hf]);
       const float inv = 1.0f / l_run[hf];
       if (EXT) {
@@ -532,10 +536,10 @@ attention_kernel(const AParams p, const __grid_constant__ CUtensorMap tm_k, cons
         for (int i = 0; i < D / 8; ++i)
 #pragma unroll
           for (int e = 0; e < 2; ++e)
-            store_ext(p, (size_t)b * p.s_new + row, head, i * 8 + 2 * t + e, o[i][hf * 2 + e] * inv);
+            store_ext(p, (size_t)(q_row + r), head, i * 8 + 2 * t + e, o[i][hf * 2 + e] * inv);
         continue;
       }
-      bf16* dst = p.out + (((size_t)b * p.s_new + row) * p.q_heads + head) * D;
+      bf16* dst = p.out + ((size_t)(q_row + r) * p.q_heads + head) * D;
 #pragma unroll
       for (int i = 0; i < D / 8; ++i)
         *reinterpret_cast<uint32_t*>(dst + i * 8 + 2 * t) = pack_bf16(o[i][hf * 2] * inv, o[i][hf * 2 + 1] * inv);
@@ -778,8 +782,9 @@ bool attention_mma_takes(const rb_kv_cache* c, int q_heads) {
 }
 
 int attention_mma_bf16(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, int s_new, int q_heads,
-                       float scale, void* out, const AttnExtra* ext) {
+                       float scale, void* out, const AttnExtra* ext, const Packed* pk) {
   AParams p{};
+  if (pk) p.start = pk->start;
   const size_t loff = (size_t)layer * c->layer_stride_elems();
   p.q = (const bf16*)q;
   p.k = (const bf16*)c->k + loff;
@@ -800,7 +805,7 @@ int attention_mma_bf16(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, in
              "attention: %d query heads per KV head unsupported (1..16)", p.group);
   // prefill with at least one 128-row query tile and head size 64 or 128: the tcgen05 kernel
   if (ctx->attn_tc && attention_prefill_tc_supported(c, s_new, q_heads, q, out, ext != nullptr))
-    return attention_prefill_tc(ctx, q, c, layer, batch, s_new, q_heads, scale, out, ext);
+    return attention_prefill_tc(ctx, q, c, layer, batch, s_new, q_heads, scale, out, ext, pk);
   int max_len = 0;
   for (int b = 0; b < batch; ++b) max_len = std::max(max_len, c->host_lens[b]);
   if (ext) {

@@ -72,6 +72,7 @@ __device__ __forceinline__ float ex2_fast(float x) {
 struct TParams {
   const int32_t* block_table;
   const int32_t* seq_lens;
+  const int32_t* start;   // Packed::start, or NULL
   int pages_per_seq, s_new, q_heads, kv_heads, group, window;
   float scale_log2;
   bf16* out;
@@ -171,15 +172,17 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
   const int q0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * kBM;  // longest causal ranges first
   const int head = blockIdx.y, b = blockIdx.z, kvh = head / p.group;
   const int len = p.seq_lens[b];
-  const int base = len - p.s_new;  // absolute position of query row 0
+  const int s_new = rows_of(p.start, b, p.s_new);
+  const int q_row = first_row(p.start, b, p.s_new) + q0;  // of q and out
+  const int base = len - s_new;  // absolute position of query row 0
   // Key tiles this CTA walks.  The window term acts among the tokens of one call only (qwen2.rs:316-334), so whole
   // tiles can be skipped only when nothing is cached.
   const int tile_lo = EXT ? first_visible(base + q0, p.x_window, p.x_chunk) / kBN : base == 0 ? max(0, q0 - p.window) / kBN : 0;
   const int tile_hi = (min(base + q0 + kBM, len) + kBN - 1) / kBN;
-  const int n = tile_hi - tile_lo;
+  const int n = q0 < s_new ? tile_hi - tile_lo : 0;  // (a ragged batch: the grid is made for its longest sequence)
   // The tiles must sit on a 1024-byte boundary (swizzle atoms); nothing else lives in shared memory before them.
   const bool layout_ok = (ptx::smem_u32(smem) & 1023u) == 0u && n >= 1;
-  if (!layout_ok && threadIdx.x == 0) { p.status[0] = (uint32_t)(-RB_ERR_CUDA); p.status[1] = 0xA7C0u; p.status[2] = blockIdx.x; }
+  if (!layout_ok && q0 < s_new && threadIdx.x == 0) { p.status[0] = (uint32_t)(-RB_ERR_CUDA); p.status[1] = 0xA7C0u; p.status[2] = blockIdx.x; }
 
   if (layout_ok && warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -187,7 +190,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
       ptx::mbar_expect_tx(&ctl->q_full, C::kQBytes);
 #pragma unroll
       for (int cb = 0; cb < C::kBlocks; ++cb)
-        ptx::tma_load_2d(q_s + cb * (kBM * 128), &tm_q, &ctl->q_full, head * D + cb * 64, b * p.s_new + q0);
+        ptx::tma_load_2d(q_s + cb * (kBM * 128), &tm_q, &ctl->q_full, head * D + cb * 64, q_row);
       bool ok = true;
       for (int j = 0; j < n && ok; ++j) {
         const int st = j & 1, kst = j % KR;
@@ -425,20 +428,20 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
       ptx::tc_fence_after();
       if (EXT && p.x_sink) l_run += ex2_fast(fmaf(__bfloat162float(p.x_sink[head]), kLog2e, -m_run));
       float inv = 1.0f / l_run;
-      const bool store = q0 + row < p.s_new;
+      const bool store = q0 + row < s_new;
       if (EXT) {
         inv *= p.x_out_scale;
         if (p.x_head_gate && store)
-          inv *= sigmoid_f(__bfloat162float(p.x_gate[((size_t)b * p.s_new + q0 + row) * p.x_gate_ld + head]));
+          inv *= sigmoid_f(__bfloat162float(p.x_gate[(size_t)(q_row + row) * p.x_gate_ld + head]));
       }
-      bf16* dst = p.out + (((size_t)b * p.s_new + q0 + row) * p.q_heads + head) * D;
+      bf16* dst = p.out + ((size_t)(q_row + row) * p.q_heads + head) * D;
 #pragma unroll 1
       for (int c0 = 0; c0 < D; c0 += 32) {
         uint32_t r[32];
         ptx::tmem_ld_32x32(t_row + C::kOCol + (uint32_t)c0, r);
         ptx::tmem_wait_ld();
         if (EXT && store) {
-          const size_t m = (size_t)b * p.s_new + q0 + row;
+          const size_t m = (size_t)(q_row + row);
           const int vd = p.x_value_dim, col0 = head * vd;
           bf16* xo = p.out + m * p.x_out_ld + col0;
           const bf16* xg = p.x_gate && !p.x_head_gate ? p.x_gate + m * p.x_gate_ld + col0 : nullptr;
@@ -504,14 +507,14 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
 
 template <int D, int EXT>
 int launch_tc(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, int s_new, int q_heads, float scale, void* out,
-              const AttnExtra* ext) {
+              const AttnExtra* ext, const Packed* pk) {
   using C = TCfg<D, EXT == 2>;
   const size_t loff = (size_t)layer * c->layer_stride_elems();
   const bf16* kbase = (const bf16*)c->k + loff;
   const bf16* vbase = (const bf16*)c->v + loff;
   CUtensorMap tq, tk, tv;
   // q rows are (sequence, position), columns (head, lane): 128-row x 64-column boxes
-  RB_TRY(tmap_2d_bf16(ctx, q, (int64_t)batch * s_new, (int64_t)q_heads * D, (int64_t)q_heads * D, kBM, &tq));
+  RB_TRY(tmap_2d_bf16(ctx, q, pk ? pk->rows : (int64_t)batch * s_new, (int64_t)q_heads * D, (int64_t)q_heads * D, kBM, &tq));
   // one map per layer and operand: rows are (page, KV head, token), 64-row x 64-column boxes
   const int64_t rows = (int64_t)c->num_pages * c->kv_heads * kBN;
   RB_TRY(tmap_2d_bf16(ctx, kbase, rows, D, D, kBN, &tk));
@@ -523,6 +526,7 @@ int launch_tc(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, 
   TParams p{};
   p.block_table = c->block_table;
   p.seq_lens = c->seq_lens;
+  p.start = pk ? pk->start : nullptr;
   p.pages_per_seq = c->pages_per_seq;
   p.s_new = s_new;
   p.q_heads = q_heads;
@@ -587,16 +591,16 @@ bool attention_prefill_tc_supported(const rb_kv_cache* c, int s_new, int q_heads
 }
 
 int attention_prefill_tc(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, int s_new, int q_heads, float scale,
-                         void* out, const AttnExtra* ext) {
+                         void* out, const AttnExtra* ext, const Packed* pk) {
   const int kind = !ext ? 0 : c->shared() ? 2 : 1;
   auto go = [&](auto plain, auto extra, auto shared) {
-    return (kind == 0 ? plain : kind == 1 ? extra : shared)(ctx, q, c, layer, batch, s_new, q_heads, scale, out, ext);
+    return (kind == 0 ? plain : kind == 1 ? extra : shared)(ctx, q, c, layer, batch, s_new, q_heads, scale, out, ext, pk);
   };
   if (c->head_dim == 64) return go(launch_tc<64, 0>, launch_tc<64, 1>, launch_tc<64, 2>);
   if (c->head_dim == 128) return go(launch_tc<128, 0>, launch_tc<128, 1>, launch_tc<128, 2>);
-  if (kind == 0 && c->head_dim == 80) return launch_tc<80, 0>(ctx, q, c, layer, batch, s_new, q_heads, scale, out, ext);
-  if (kind == 0 && c->head_dim == 96) return launch_tc<96, 0>(ctx, q, c, layer, batch, s_new, q_heads, scale, out, ext);
-  if (kind == 0 && c->head_dim == 256) return launch_tc<256, 0>(ctx, q, c, layer, batch, s_new, q_heads, scale, out, ext);
+  if (kind == 0 && c->head_dim == 80) return launch_tc<80, 0>(ctx, q, c, layer, batch, s_new, q_heads, scale, out, ext, pk);
+  if (kind == 0 && c->head_dim == 96) return launch_tc<96, 0>(ctx, q, c, layer, batch, s_new, q_heads, scale, out, ext, pk);
+  if (kind == 0 && c->head_dim == 256) return launch_tc<256, 0>(ctx, q, c, layer, batch, s_new, q_heads, scale, out, ext, pk);
   return fail(RB_ERR_UNIMPLEMENTED, "tensor-core prefill attention: head_dim %d unsupported", c->head_dim);
 }
 

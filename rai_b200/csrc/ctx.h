@@ -293,8 +293,22 @@ __device__ __forceinline__ float tanh_sfu(float x) {
 // slope of the distance bias, 2^(-8 (h + 1) / heads)
 __device__ __forceinline__ float alibi_slope(int head, int heads) { return exp2f(-8.0f * (float)(head + 1) / (float)heads); }
 
+// The rows of a ragged call without its padding: sequence b's rows are [start[b], start[b + 1]) (device arrays; s_new is then the
+// longest sequence's count, and the cache's lengths end with the last real row).
+struct Packed {
+  const int32_t* start = nullptr;  // [batch + 1]
+  const int32_t* seq = nullptr;    // [rows]: the sequence a row belongs to
+  int rows = 0;
+};
+__device__ __forceinline__ int rows_of(const int32_t* start, int b, int s_new) { return start ? start[b + 1] - start[b] : s_new; }
+__device__ __forceinline__ int first_row(const int32_t* start, int b, int s_new) { return start ? start[b] : b * s_new; }
+// decoder_kernels.cu, api.cu: rb_rope_kv_append and rb_attention over packed rows (pk NULL: batch x s_new of them)
+int rope_kv_append(rb_ctx* ctx, const void* qkv, const float* acc, int n_acc, const void* bias, const float* cos_t, const float* sin_t,
+                   int rot, int batch, int s_new, int q_heads, rb_kv_cache* c, int layer, void* q_out, int dtype, const Packed* pk);
+int attention_rows(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, int s_new, int q_heads, float scale, void* out,
+                   int dtype, const Packed* pk);
 int attention_mma_bf16(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, int s_new, int q_heads,
-                       float scale, void* out, const AttnExtra* ext = nullptr);
+                       float scale, void* out, const AttnExtra* ext = nullptr, const Packed* pk = nullptr);
 bool attention_mma_takes(const rb_kv_cache* c, int q_heads);
 // decoder_kernels.cu: the tensor-parallel sum of a row-parallel product (split-K slabs + bias, or a finished bf16
 // tensor `part`) over the exchange buffers, the residual add and the following norm, in one kernel.
@@ -322,7 +336,7 @@ int attention_reserve_scratch(rb_ctx* ctx, size_t bytes);
 // attention_tc.cu: causal prefill attention on tcgen05 (head sizes 64 and 128, without `extra` also 80, 96 and 256; query length >= 128)
 bool attention_prefill_tc_supported(const rb_kv_cache* c, int s_new, int q_heads, const void* q, const void* out, bool extra);
 int attention_prefill_tc(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, int s_new, int q_heads, float scale,
-                         void* out, const AttnExtra* ext = nullptr);
+                         void* out, const AttnExtra* ext = nullptr, const Packed* pk = nullptr);
 // attention_latent.cu, attention_talk.cu: attention with mixed heads or over latents, one block for all heads of its tokens
 bool attention_joint_takes(const rb_kv_cache* c, const AttnExtra& x);
 int attention_joint_row_tiles(const rb_kv_cache* c, int q_heads);   // blocks a single token's heads take
@@ -336,5 +350,5 @@ int attention_mix_tc(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int 
 int attention_talk_simple(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, int s_new, int q_heads, float scale, void* out,
                           int dtype, const AttnExtra& x);
 int attention_simple(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, int s_new, int q_heads,
-                     float scale, void* out, int dtype, const AttnExtra* ext = nullptr);
+                     float scale, void* out, int dtype, const AttnExtra* ext = nullptr, const Packed* pk = nullptr);
 }  // namespace rb

@@ -586,14 +586,14 @@ __global__ void rope_kv_append_kernel(const T* __restrict__ qkv, const float* __
                                       int s_new, int q_heads, int kv_heads, int d, T* __restrict__ q_out,
                                       T* __restrict__ k_cache, T* __restrict__ v_cache,
                                       const int32_t* __restrict__ block_table, const int32_t* __restrict__ seq_lens,
-                                      int pages_per_seq, int max_seq, uint32_t* status) {
+                                      int pages_per_seq, int max_seq, uint32_t* status, const Packed pk) {
   extern __shared__ float vals[];  // all (q + 2 kv) * d columns of this token
   pdl_launch_dependents();
   pdl_wait();
   const int m = blockIdx.x;
-  const int b = m / s_new, s = m % s_new;
+  const int b = pk.seq ? pk.seq[m] : m / s_new;
   const int ncol = (q_heads + 2 * kv_heads) * d;
-  const int pos = seq_lens[b] - s_new + s;
+  const int pos = seq_lens[b] - rows_of(pk.start, b, s_new) + m - first_row(pk.start, b, s_new);
   if (pos < 0 || pos >= max_seq) {
     if (threadIdx.x == 0) { status[0] = (uint32_t)(-RB_ERR_INVALID); status[1] = 0x20BEu; status[2] = (uint32_t)pos; }
     return;
@@ -642,13 +642,13 @@ __global__ void rope_kv_append_vec_kernel(const T* __restrict__ qkv, const float
                                           T* __restrict__ k_cache, T* __restrict__ v_cache,
                                           const int32_t* __restrict__ block_table,
                                           const int32_t* __restrict__ seq_lens, int pages_per_seq, int max_seq,
-                                          uint32_t* status) {
+                                          uint32_t* status, const Packed pk) {
   pdl_launch_dependents();
   pdl_wait();
   const int m = blockIdx.x;
-  const int b = m / s_new, sq = m % s_new;
+  const int b = pk.seq ? pk.seq[m] : m / s_new;
   const int ncol = (q_heads + 2 * kv_heads) * d;
-  const int pos = seq_lens[b] - s_new + sq;
+  const int pos = seq_lens[b] - rows_of(pk.start, b, s_new) + m - first_row(pk.start, b, s_new);
   if (pos < 0 || pos >= max_seq) {
     if (threadIdx.x == 0) { status[0] = (uint32_t)(-RB_ERR_INVALID); status[1] = 0x20BEu; status[2] = (uint32_t)pos; }
     return;
@@ -1017,9 +1017,9 @@ extern "C" int32_t rb_rope_tables(rb_ctx* ctx, int32_t recipe, int32_t rot_dim, 
 template <typename T>
 static int rope_launch(rb_ctx* ctx, const void* qkv, const float* acc, int n_acc, const void* bias, const float* cos_t,
                        const float* sin_t, int rot, int batch, int s_new, int q_heads, rb_kv_cache* c, int layer,
-                       void* q_out) {
-  const int d = c->head_dim, ncol = (q_heads + 2 * c->kv_heads) * d;
-  const size_t acc_stride = (size_t)batch * s_new * ncol;
+                       void* q_out, const Packed* pk) {
+  const int d = c->head_dim, ncol = (q_heads + 2 * c->kv_heads) * d, rows = pk ? pk->rows : batch * s_new;
+  const size_t acc_stride = (size_t)rows * ncol;
   const size_t loff = (size_t)layer * c->layer_stride_elems();
   T* kc = (T*)c->k + loff;
   T* vc = (T*)c->v + loff;
@@ -1029,25 +1029,30 @@ static int rope_launch(rb_ctx* ctx, const void* qkv, const float* acc, int n_acc
   if (vec_ok) {
     const int items = (q_heads + c->kv_heads) * (half / 8 + (d - rot) / 8) + c->kv_heads * (d / 8);
     const int threads = std::min(512, (items + 31) / 32 * 32);
-    RB_CUDA(launch_kernel(rope_kv_append_vec_kernel<T>, dim3((unsigned)(batch * s_new)), dim3(threads), 0, ctx->stream,
+    RB_CUDA(launch_kernel(rope_kv_append_vec_kernel<T>, dim3((unsigned)rows), dim3(threads), 0, ctx->stream,
                           ctx->pdl, (const T*)qkv, acc, n_acc, acc_stride, (const T*)bias, cos_t, sin_t, rot, s_new,
                           q_heads, c->kv_heads, d, (T*)q_out, kc, vc, (const int32_t*)c->block_table,
-                          (const int32_t*)c->seq_lens, c->pages_per_seq, c->max_seq, ctx->status_dev));
+                          (const int32_t*)c->seq_lens, c->pages_per_seq, c->max_seq, ctx->status_dev, pk ? *pk : Packed()));
     return RB_OK;
   }
   const size_t smem = (size_t)ncol * sizeof(float);
   auto kern = rope_kv_append_kernel<T>;
   if (smem > 48 * 1024) RB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  RB_CUDA(launch_kernel(kern, dim3((unsigned)(batch * s_new)), dim3(256), smem, ctx->stream, ctx->pdl, (const T*)qkv, acc,
+  RB_CUDA(launch_kernel(kern, dim3((unsigned)rows), dim3(256), smem, ctx->stream, ctx->pdl, (const T*)qkv, acc,
                         n_acc, acc_stride, (const T*)bias, cos_t, sin_t, rot, s_new, q_heads, c->kv_heads, d, (T*)q_out,
                         kc, vc, (const int32_t*)c->block_table, (const int32_t*)c->seq_lens, c->pages_per_seq,
-                        c->max_seq, ctx->status_dev));
+                        c->max_seq, ctx->status_dev, pk ? *pk : Packed()));
   return RB_OK;
 }
 
 extern "C" int32_t rb_rope_kv_append(rb_ctx* ctx, const void* qkv, const float* acc, int32_t n_acc, const void* bias,
                                      const float* cos_t, const float* sin_t, int32_t rot, int32_t batch, int32_t s_new,
                                      int32_t q_heads, rb_kv_cache* c, int32_t layer, void* q_out, int32_t dtype) {
+  return rope_kv_append(ctx, qkv, acc, n_acc, bias, cos_t, sin_t, rot, batch, s_new, q_heads, c, layer, q_out, dtype, nullptr);
+}
+
+int rb::rope_kv_append(rb_ctx* ctx, const void* qkv, const float* acc, int n_acc, const void* bias, const float* cos_t, const float* sin_t,
+                       int rot, int batch, int s_new, int q_heads, rb_kv_cache* c, int layer, void* q_out, int dtype, const Packed* pk) {
   RB_REQUIRE(ctx && c && q_out && cos_t && sin_t, "rb_rope_kv_append: null argument");
   RB_REQUIRE(qkv || (acc && n_acc > 0), "rb_rope_kv_append: no input given");
   RB_REQUIRE(dtype == c->dtype, "rb_rope_kv_append: cache dtype differs");
@@ -1057,11 +1062,11 @@ extern "C" int32_t rb_rope_kv_append(rb_ctx* ctx, const void* qkv, const float* 
   if (!acc) n_acc = 0;
   if (n_acc == 0) acc = nullptr;
   const int ncol = (q_heads + 2 * c->kv_heads) * c->head_dim;
-  ProfScope prof(ctx, RB_PROF_ROPE_KV, (double)batch * s_new * ncol * (dtype_size(dtype) * (qkv ? 2.0 : 1.0) + 4.0 * n_acc), 0.0);
+  ProfScope prof(ctx, RB_PROF_ROPE_KV, (double)(pk ? pk->rows : batch * s_new) * ncol * (dtype_size(dtype) * (qkv ? 2.0 : 1.0) + 4.0 * n_acc), 0.0);
   if (dtype == RB_BF16)
-    RB_TRY(rope_launch<__nv_bfloat16>(ctx, qkv, acc, n_acc, bias, cos_t, sin_t, rot, batch, s_new, q_heads, c, layer, q_out));
+    RB_TRY(rope_launch<__nv_bfloat16>(ctx, qkv, acc, n_acc, bias, cos_t, sin_t, rot, batch, s_new, q_heads, c, layer, q_out, pk));
   else if (dtype == RB_F32)
-    RB_TRY(rope_launch<float>(ctx, qkv, acc, n_acc, bias, cos_t, sin_t, rot, batch, s_new, q_heads, c, layer, q_out));
+    RB_TRY(rope_launch<float>(ctx, qkv, acc, n_acc, bias, cos_t, sin_t, rot, batch, s_new, q_heads, c, layer, q_out, pk));
   else
     return fail(RB_ERR_DTYPE, "rb_rope_kv_append: dtype %d unsupported", dtype);
   ctx->launches++;

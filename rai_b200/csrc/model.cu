@@ -113,6 +113,14 @@ __global__ void gather_rows_kernel(const uint4* __restrict__ src, const int32_t*
   for (int i = threadIdx.x; i < pieces_per_row; i += blockDim.x) dst[(size_t)b * pieces_per_row + i] = src[r * pieces_per_row + i];
 }
 
+// ids of the real tokens of a ragged call
+__global__ void pack_ids_kernel(const uint32_t* __restrict__ tokens, int seq, const Packed pk, uint32_t* __restrict__ out) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= pk.rows) return;
+  const int b = pk.seq[r];
+  out[r] = tokens[(size_t)b * seq + r - pk.start[b]];
+}
+
 // out[b, r*vl + j] = gathered[r, b, j]  (vocabulary shards back into rows of logits)
 template <typename T>
 __global__ void unshard_logits_kernel(const T* __restrict__ g, T* __restrict__ out, int tp, int batch, int vl) {
@@ -286,7 +294,7 @@ int last_rows_logits(rb_model* m, int seq, const int32_t* rows_dev, int n) {
 }
 
 int forward_body(rb_model* m, const uint32_t* tokens, int batch, int seq, void* logits_out, const int32_t* rows_dev = nullptr,
-                 int n_rows = -1, const int32_t* new_lens = nullptr);
+                 int n_rows = -1, const int32_t* new_lens = nullptr, const Packed* pk = nullptr);
 int finish_logits(rb_model* m, int batch, int seq, void* logits_out, const int32_t* rows_dev, int n_rows);
 
 // act = activation(x . W1^T [+ b1]) [* (x . Wup^T)]  -- the first half of MLP::fwd.  When the fused kernel
@@ -344,8 +352,9 @@ int forward_impl(rb_model* m, const uint32_t* tokens, int batch, int seq, int po
 // cache's sequence lengths), so the same sequence of launches serves every decode step.
 // Logits are computed for rows_dev[0..n_rows) of the call, or (rows_dev == NULL) for the last position of each sequence.
 // new_lens (device, NULL = seq each): how many of a sequence's rows are tokens; the rest is padding.
+// pk (not for layered designs): the call's rows are packed, tokens and rows_dev name packed rows, seq is the longest count.
 int forward_body(rb_model* m, const uint32_t* tokens, int batch, int seq, void* logits_out, const int32_t* rows_dev, int n_rows,
-                 const int32_t* new_lens) {
+                 const int32_t* new_lens, const Packed* pk) {
   if (!rows_dev) n_rows = batch;
   if (m->layered) {
     RB_TRY(layered_forward(m, tokens, batch, seq, new_lens));
@@ -355,7 +364,7 @@ int forward_body(rb_model* m, const uint32_t* tokens, int batch, int seq, void* 
   rb_ctx* ctx = m->ctx;
   RB_REQUIRE(c.tp_size == 1 || m->comm || m->shard_only,
              "forward: this is rank %d of a %d-way tensor-parallel model and rb_model_tp_init has not run", c.tp_rank, c.tp_size);
-  const int64_t rows = (int64_t)batch * seq;
+  const int64_t rows = pk ? pk->rows : (int64_t)batch * seq;
   const int H = c.hidden_size, d = m->d;
   m->xchg_index = 0;
 
@@ -373,23 +382,23 @@ int forward_body(rb_model* m, const uint32_t* tokens, int batch, int seq, void* 
     int s = 1;
     if (use_partials(m, rows, m->nqkv_l, H, &s)) {
       RB_TRY(rb_linear_partials(ctx, m->xn, w.qkv, m->scratch, rows, m->nqkv_l, H, s));
-      if (seq == 1) {  // single-token step: RoPE and the cache append ride in the attention kernel when they can
+      if (seq == 1 && !pk) {  // single-token step: RoPE and the cache append ride in the attention kernel when they can
         RB_TRY(rb_rope_attention_decode(ctx, nullptr, m->scratch, s, w.qkv_b, m->rope_cos, m->rope_sin, c.rotary_dim, batch,
                                         m->nq_l, m->cache, l, scale, m->q, m->attn, c.dtype));
       } else {
-        RB_TRY(rb_rope_kv_append(ctx, nullptr, m->scratch, s, w.qkv_b, m->rope_cos, m->rope_sin, c.rotary_dim, batch, seq,
-                                 m->nq_l, m->cache, l, m->q, c.dtype));
-        RB_TRY(rb_attention(ctx, m->q, m->cache, l, batch, seq, m->nq_l, scale, m->attn, c.dtype));
+        RB_TRY(rope_kv_append(ctx, nullptr, m->scratch, s, w.qkv_b, m->rope_cos, m->rope_sin, c.rotary_dim, batch, seq,
+                              m->nq_l, m->cache, l, m->q, c.dtype, pk));
+        RB_TRY(attention_rows(ctx, m->q, m->cache, l, batch, seq, m->nq_l, scale, m->attn, c.dtype, pk));
       }
     } else {
       RB_TRY(rb_linear(ctx, m->xn, w.qkv, w.qkv_b, nullptr, m->qkv, rows, m->nqkv_l, H, RB_ACT_NONE, c.dtype));
-      if (seq == 1) {
+      if (seq == 1 && !pk) {
         RB_TRY(rb_rope_attention_decode(ctx, m->qkv, nullptr, 0, nullptr, m->rope_cos, m->rope_sin, c.rotary_dim, batch,
                                         m->nq_l, m->cache, l, scale, m->q, m->attn, c.dtype));
       } else {
-        RB_TRY(rb_rope_kv_append(ctx, m->qkv, nullptr, 0, nullptr, m->rope_cos, m->rope_sin, c.rotary_dim, batch, seq,
-                                 m->nq_l, m->cache, l, m->q, c.dtype));
-        RB_TRY(rb_attention(ctx, m->q, m->cache, l, batch, seq, m->nq_l, scale, m->attn, c.dtype));
+        RB_TRY(rope_kv_append(ctx, m->qkv, nullptr, 0, nullptr, m->rope_cos, m->rope_sin, c.rotary_dim, batch, seq,
+                              m->nq_l, m->cache, l, m->q, c.dtype, pk));
+        RB_TRY(attention_rows(ctx, m->q, m->cache, l, batch, seq, m->nq_l, scale, m->attn, c.dtype, pk));
       }
     }
     RB_TRY(linear_into_residual(m, pend, m->attn, w.o, w.o_b, rows, H, (int64_t)m->nq_l * d));
@@ -709,6 +718,8 @@ extern "C" int32_t rb_model_create(rb_ctx* ctx, const rb_model_config* cfg, rb_m
   W((size_t)c.max_batch * V * m->es, &m->logits);
   if (tp > 1) W((size_t)c.max_batch * Vl * m->es * (tp + 1), &m->logits_g);
   W((size_t)c.max_batch * sizeof(uint32_t), (void**)&m->next_ids);
+  W((2 * MT + c.max_batch + 1) * sizeof(int32_t), (void**)&m->pack);
+  W(MT * sizeof(uint32_t), (void**)&m->pack_ids);
   W(MT * sizeof(int32_t), (void**)&m->last_rows);
   W((size_t)c.max_batch * sizeof(int32_t), (void**)&m->new_lens);
   if (c.dtype == RB_BF16) {
@@ -1045,6 +1056,32 @@ static int forward_rows(rb_model* m, const uint32_t* tokens, int batch, int seq,
     RB_CUDA(cudaMemcpyAsync(m->new_lens, m->new_lens_host.data(), (size_t)batch * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
   }
   const std::vector<int32_t> before(kc->host_lens.begin(), kc->host_lens.begin() + batch);
+  if (lens && !m->layered && seq > 1) {
+    // Padding is left out of the call unless somebody wants the logits of a padding row: sequence b's tokens become rows
+    // start[b], start[b] + 1, ... of every product, and its new keys and values are those of its tokens alone.
+    Packed pk;
+    std::vector<int32_t>& h = m->pack_host;
+    h.assign((size_t)batch + 1, 0);
+    for (int b = 0; b < batch; ++b) h[b + 1] = h[b] + lens[b];
+    pk.rows = h[batch];
+    bool real = pk.rows > 0 && pk.rows < total;
+    for (int i = 0; real && i < n_rows; ++i) real = rows[i] % seq < lens[rows[i] / seq];
+    if (real) {
+      for (int b = 0; b < batch; ++b) h.insert(h.end(), (size_t)lens[b], b);
+      for (int i = 0; i < n_rows; ++i) h.push_back(h[rows[i] / seq] + rows[i] % seq);
+      RB_CUDA(cudaMemcpyAsync(m->pack, h.data(), h.size() * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
+      pk.start = m->pack;
+      pk.seq = m->pack + batch + 1;
+      pack_ids_kernel<<<(pk.rows + 255) / 256, 256, 0, ctx->stream>>>(tokens, seq, pk, m->pack_ids);
+      RB_CUDA(cudaGetLastError());
+      ctx->launches++;
+      for (int b = 0; b < batch; ++b) kc->host_lens[b] = before[b] + lens[b];
+      RB_CUDA(cudaMemcpyAsync(kc->seq_lens, kc->host_lens.data(), (size_t)batch * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
+      // (at least 2: a count of 1 would mean one row for every sequence)
+      const int longest = std::max(2, *std::max_element(lens, lens + batch));
+      return forward_body(m, m->pack_ids, batch, longest, logits_out, pk.seq + pk.rows, n_rows, nullptr, &pk);
+    }
+  }
   for (int b = 0; b < batch; ++b) kc->host_lens[b] = before[b] + seq;
   RB_CUDA(cudaMemcpyAsync(kc->seq_lens, kc->host_lens.data(), (size_t)batch * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
   const int st = forward_body(m, tokens, batch, seq, logits_out, m->last_rows, n_rows, lens ? m->new_lens : nullptr);

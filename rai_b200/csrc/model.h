@@ -92,6 +92,10 @@ struct rb_model {
   int64_t params_loaded = 0;   // grows with every parameter that is loaded
   // workspace
   uint32_t* ids = nullptr;
+  // a ragged call without its padding: [batch + 1] first rows, [rows] sequences, the rows whose logits are wanted; its token ids
+  int32_t* pack = nullptr;
+  uint32_t* pack_ids = nullptr;
+  std::vector<int32_t> pack_host;         // outlives the asynchronous upload
   void *h = nullptr, *xn = nullptr, *tmp = nullptr, *qkv = nullptr, *q = nullptr, *attn = nullptr, *act = nullptr;
   void *last_h = nullptr, *logits = nullptr, *logits_g = nullptr;
   uint32_t* next_ids = nullptr;

@@ -76,12 +76,13 @@ __global__ void __launch_bounds__(kPlainAttnWarps * 32)
 attention_plain_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
                        const int32_t* __restrict__ block_table, const int32_t* __restrict__ seq_lens, int pages_per_seq,
                        int s_new, int q_heads, int kv_heads, int d, float scale, int window, T* __restrict__ out, int ext,
-                       const AttnExtra x) {
+                       const AttnExtra x, const Packed pk) {
   __shared__ float sm_m[kPlainAttnWarps], sm_l[kPlainAttnWarps], sm_o[kPlainAttnWarps][32 * NJ];
   const int m = blockIdx.x, h = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = m / s_new, s = m % s_new;
-  const int limit = seq_lens[b] - s_new + s;  // last visible key
+  const int b = pk.seq ? pk.seq[m] : m / s_new;
+  const int call_base = seq_lens[b] - rows_of(pk.start, b, s_new);  // first token of this call
+  const int limit = call_base + m - first_row(pk.start, b, s_new);  // last visible key
   const int kvh = h / (q_heads / kv_heads);
   float qv[NJ], o[NJ];
 #pragma unroll
@@ -91,7 +92,6 @@ attention_plain_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, c
     o[j] = 0.f;
   }
   float mx = -INFINITY, l = 0.f;
-  const int call_base = seq_lens[b] - s_new;  // first token of this call
   const int first = ext ? first_visible(limit, x.window > 0 ? x.window : 1 << 30, x.chunk) : 0;
   const float slope = ext && x.alibi ? alibi_slope(h, q_heads) : 0.f;
   if (ext) scale *= query_temperature(limit, x.temp_every, x.temp_coef);
@@ -271,24 +271,24 @@ int gemm_simple(rb_ctx* ctx, const GemmArgs& a, int dtype) {
 
 template <typename T, int NJ>
 static int attention_plain_launch(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, int s_new, int q_heads, float scale,
-                                  void* out, const AttnExtra* ext) {
+                                  void* out, const AttnExtra* ext, const Packed* pk) {
   const size_t loff = (size_t)layer * c->layer_stride_elems();
-  dim3 grid((unsigned)(batch * s_new), (unsigned)q_heads);
+  dim3 grid((unsigned)(pk ? pk->rows : batch * s_new), (unsigned)q_heads);
   attention_plain_kernel<T, NJ><<<grid, kPlainAttnWarps * 32, 0, ctx->stream>>>(
       (const T*)q, (const T*)c->k + loff, (const T*)c->v + loff, c->block_table, c->seq_lens, c->pages_per_seq, s_new, q_heads, c->kv_heads,
-      c->head_dim, scale, c->window, (T*)out, ext ? 1 : 0, ext ? *ext : AttnExtra());
+      c->head_dim, scale, c->window, (T*)out, ext ? 1 : 0, ext ? *ext : AttnExtra(), pk ? *pk : Packed());
   ctx->launches++;
   return launch_status("attention_plain");
 }
 
 int attention_simple(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, int s_new, int q_heads,
-                     float scale, void* out, int dtype, const AttnExtra* ext) {
+                     float scale, void* out, int dtype, const AttnExtra* ext, const Packed* pk) {
   RB_REQUIRE(dtype == RB_F32 || dtype == RB_BF16, "attention: dtype %d unsupported", dtype);
   RB_REQUIRE(c->head_dim <= 1024, "attention: head_dim %d exceeds 1024", c->head_dim);
   const bool wide = c->head_dim > 256;
   const auto run = dtype == RB_F32 ? (wide ? attention_plain_launch<float, 32> : attention_plain_launch<float, 8>)
                                    : (wide ? attention_plain_launch<__nv_bfloat16, 32> : attention_plain_launch<__nv_bfloat16, 8>);
-  return run(ctx, q, c, layer, batch, s_new, q_heads, scale, out, ext);
+  return run(ctx, q, c, layer, batch, s_new, q_heads, scale, out, ext, pk);
 }
 
 template <typename T>

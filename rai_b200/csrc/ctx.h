@@ -178,6 +178,18 @@ struct GemmArgs {
 };
 int gemm_tc_bf16(rb_ctx* ctx, const GemmArgs& a);
 int gemm_pair_bf16(rb_ctx* ctx, const GemmArgs& a);   // gemm_pair.cu: M > 256, no partials
+// gemm_rows.cu: a bf16 product of at most eight rows with everything around it: rows are normalised first (norm: a kind, -1: no);
+// out = act(product + bias) + residual, act(product) * up product, or the plain sums as out_f
+struct RowsArgs {
+  const void *x = nullptr, *norm_w = nullptr, *norm_b = nullptr, *w = nullptr, *w2 = nullptr, *bias = nullptr, *residual = nullptr;
+  void* out = nullptr;
+  float* out_f = nullptr;
+  int64_t m = 0, n = 0, k = 0;
+  int act = RB_ACT_NONE, norm = -1;
+  float eps = 0.f;
+};
+bool gemm_rows_takes(int64_t m, int64_t k, bool norm);
+int gemm_rows(rb_ctx* ctx, const RowsArgs& a);
 constexpr int kMaxExperts = 256;
 int gemm_tc_grouped(rb_ctx* ctx, const GemmArgs& a);
 bool grouped_wants_sorted(int64_t rows, int top, int experts);

@@ -330,6 +330,53 @@ int mlp_up(rb_model* m, const LayerW& w, int64_t rows) {
   return rb_linear(ctx, m->xn, w.gate, w.fc1_b, nullptr, m->act, rows, m->inter_l, H, c.hidden_act, c.dtype);
 }
 
+// Whether a layer of so few rows takes the kernels that fold norms and residual sums into the products.
+bool few_rows(const rb_model* m, int64_t rows) {
+  const rb_model_config& c = m->cfg;
+  // Worth it where a layer's launches, not its bytes, are most of its time.  us per step, with the kernels for more rows -> these:
+  // 30 MB of weights a layer 1036 -> 651 (one row), 1058 -> 850 (eight); 157 MB 2035 -> 1959, 2212 -> 2206; 226 MB 2217 -> 2130 but,
+  // with four rows, 2821 -> 3083; 466 MB 3062 -> 3483.
+  const int64_t layer_weights = (int64_t)c.hidden_size * (m->nqkv_l + (int64_t)m->nq_l * m->d + (c.arch == RB_ARCH_PHI2 ? 2 : 3) * (int64_t)m->inter_l);
+  if (layer_weights * 2 > (96 << 20)) return false;
+  return c.dtype == RB_BF16 && c.tp_size == 1 && !m->ctx->debug_simple && !m->ctx->debug_simple_gemm && c.hidden_act != RB_ACT_XIELU &&
+         (size_t)rows * m->nqkv_l <= m->scratch_floats && gemm_rows_takes(rows, c.hidden_size, true) &&
+         gemm_rows_takes(rows, (int64_t)m->nq_l * m->d, false) && gemm_rows_takes(rows, m->inter_l, false);
+}
+
+// One layer of at most eight rows: five launches (see gemm_rows.cu).
+int few_rows_layer(rb_model* m, const LayerW& w, int l, int batch, int seq, int64_t rows, float scale, const Packed* pk) {
+  const rb_model_config& c = m->cfg;
+  rb_ctx* ctx = m->ctx;
+  const bool phi2 = c.arch == RB_ARCH_PHI2;
+  RowsArgs in;                       // from the normalised stream
+  in.x = m->h; in.m = rows; in.k = c.hidden_size; in.norm = norm_kind(m); in.eps = (float)c.norm_eps;
+  in.norm_w = w.ln1_w; in.norm_b = w.ln1_b;
+  RowsArgs qkv = in, up = in;
+  qkv.w = w.qkv; qkv.n = m->nqkv_l; qkv.out_f = m->scratch;
+  up.w = w.gate; up.w2 = phi2 ? nullptr : w.up; up.bias = phi2 ? w.fc1_b : nullptr; up.n = m->inter_l; up.act = c.hidden_act; up.out = m->act;
+  if (!phi2) { up.norm_w = w.ln2_w; up.norm_b = nullptr; }
+  RowsArgs o, down;                  // into the stream
+  o.x = m->attn; o.w = w.o; o.bias = w.o_b; o.k = (int64_t)m->nq_l * m->d;
+  down.x = m->act; down.w = w.down; down.bias = w.down_b; down.k = m->inter_l;
+  o.m = down.m = rows; o.n = down.n = c.hidden_size;
+  o.out = down.out = m->h;
+  o.residual = down.residual = m->h;
+
+  RB_TRY(gemm_rows(ctx, qkv));
+  if (phi2) RB_TRY(gemm_rows(ctx, up));   // the MLP reads the same normed rows as attention, before that adds to them (phi2.rs:293-299)
+  if (seq == 1 && !pk) {
+    RB_TRY(rb_rope_attention_decode(ctx, nullptr, m->scratch, 1, w.qkv_b, m->rope_cos, m->rope_sin, c.rotary_dim, batch, m->nq_l, m->cache, l,
+                                    scale, m->q, m->attn, c.dtype));
+  } else {
+    RB_TRY(rope_kv_append(ctx, nullptr, m->scratch, 1, w.qkv_b, m->rope_cos, m->rope_sin, c.rotary_dim, batch, seq, m->nq_l, m->cache, l, m->q,
+                          c.dtype, pk));
+    RB_TRY(attention_rows(ctx, m->q, m->cache, l, batch, seq, m->nq_l, scale, m->attn, c.dtype, pk));
+  }
+  RB_TRY(gemm_rows(ctx, o));
+  if (!phi2) RB_TRY(gemm_rows(ctx, up));
+  return gemm_rows(ctx, down);
+}
+
 int forward_impl(rb_model* m, const uint32_t* tokens, int batch, int seq, int pos, void* logits_out) {
   const rb_model_config& c = m->cfg;
   rb_ctx* ctx = m->ctx;
@@ -374,8 +421,13 @@ int forward_body(rb_model* m, const uint32_t* tokens, int batch, int seq, void* 
   const float scale = 1.0f / sqrtf((float)d);
   const int L = c.num_hidden_layers;
   Pending pend;
+  const bool few = few_rows(m, rows);
   for (int l = 0; l < L; ++l) {
     const LayerW& w = m->layers[l];
+    if (few) {
+      RB_TRY(few_rows_layer(m, w, l, batch, seq, rows, scale, pk));
+      continue;
+    }
     // input_layernorm, folding what the previous layer left pending
     RB_TRY(norm_point(m, pend, w.ln1_w, w.ln1_b, rows, m->xn));
     // q/k/v projection -> rope -> cache

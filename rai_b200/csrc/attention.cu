@@ -759,7 +759,9 @@ int attention_decode_splits(rb_ctx* ctx, int batch, int kv_heads, int max_len, i
   // One block per (sequence, KV head) keeps its copy pipeline full and needs no merge; splitting the
   // keys only pays when those pairs under-fill the GPU.  Cost model in units of key tiles: a launch
   // runs ceil(blocks / resident blocks) waves, each as long as one block's tiles plus a fixed start-up,
-  // and a split launch pays for the merge kernel.
+  // and a split launch pays for handing its parts to whoever merges them, about six tiles (two query groups of seven heads of
+  // 64, us per step of 24 layers, split -> not: 2 tiles 744 -> 651, 5 tiles 747 -> 680, 10 tiles 782 -> 745; 8 tiles of 32 heads
+  // of 80 2053 -> 2161).
   const int tiles = std::max(1, (max_len + kTile - 1) / kTile);
   const int work = batch * kv_heads;
   const int slots = (head_dim <= 128 ? 2 : 1) * ctx->sm_count;  // blocks resident at once (head size 256: one per SM)
@@ -767,7 +769,7 @@ int attention_decode_splits(rb_ctx* ctx, int batch, int kv_heads, int max_len, i
   double best_cost = 1e30;
   for (int s = 1; s <= std::min(tiles, 32); ++s) {
     const int waves = (work * s + slots - 1) / slots;
-    const double cost = (double)waves * ((tiles + s - 1) / s + 2.0) + (s > 1 ? 1.5 : 0.0);
+    const double cost = (double)waves * ((tiles + s - 1) / s + 2.0) + (s > 1 ? 6.0 : 0.0);
     if (cost < best_cost - 1e-9) { best_cost = cost; best = s; }
   }
   static const int forced = getenv("RAI_B200_ATTN_SPLITS") ? atoi(getenv("RAI_B200_ATTN_SPLITS")) : 0;

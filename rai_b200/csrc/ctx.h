@@ -317,6 +317,9 @@ __device__ __forceinline__ int first_row(const int32_t* start, int b, int s_new)
 // decoder_kernels.cu, api.cu: rb_rope_kv_append and rb_attention over packed rows (pk NULL: batch x s_new of them)
 int rope_kv_append(rb_ctx* ctx, const void* qkv, const float* acc, int n_acc, const void* bias, const float* cos_t, const float* sin_t,
                    int rot, int batch, int s_new, int q_heads, rb_kv_cache* c, int layer, void* q_out, int dtype, const Packed* pk);
+// prompt_kernels.cu: head split and rotation of many bf16 rows with nothing to add (false: not this call)
+bool rope_prompt(rb_ctx* ctx, const void* qkv, const float* cos_t, const float* sin_t, int rot, int rows, int s_new, int q_heads, rb_kv_cache* c,
+                 void* k, void* v, void* q_out, const Packed* pk, cudaError_t* status);
 int attention_rows(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, int s_new, int q_heads, float scale, void* out,
                    int dtype, const Packed* pk);
 int attention_mma_bf16(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, int s_new, int q_heads,

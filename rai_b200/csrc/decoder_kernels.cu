@@ -6,6 +6,8 @@
 #include <algorithm>
 #include <vector>
 
+#include <type_traits>
+
 #include "ctx.h"
 
 namespace rb {
@@ -1026,6 +1028,12 @@ static int rope_launch(rb_ctx* ctx, const void* qkv, const float* acc, int n_acc
   const int half = rot / 2;
   const bool vec_ok = (d % 8) == 0 && (half % 8) == 0 && aligned16(qkv) && aligned16(acc) && aligned16(bias) &&
                       aligned16(q_out) && aligned16(cos_t) && aligned16(sin_t) && ((acc_stride * sizeof(float)) % 16) == 0;
+  cudaError_t launched = cudaSuccess;
+  if (vec_ok && std::is_same<T, __nv_bfloat16>::value && !acc && !bias &&
+      rope_prompt(ctx, qkv, cos_t, sin_t, rot, rows, s_new, q_heads, c, kc, vc, q_out, pk, &launched)) {
+    RB_CUDA(launched);
+    return RB_OK;
+  }
   if (vec_ok) {
     const int items = (q_heads + c->kv_heads) * (half / 8 + (d - rot) / 8) + c->kv_heads * (d / 8);
     const int threads = std::min(512, (items + 31) / 32 * 32);

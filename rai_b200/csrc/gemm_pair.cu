@@ -515,9 +515,12 @@ PairSpace* pair_space(rb_ctx* ctx) {
     if (s.slabs && s.stream == ctx->stream) return &s;
     if (!s.slabs) {
       if (cudaMalloc(&s.slabs, kPairSlabBytes) != cudaSuccess) { cudaGetLastError(); s.slabs = nullptr; return nullptr; }
-      if (cudaMalloc(&s.flags, kPairFlagBytes) != cudaSuccess || cudaMemset(s.flags, 0, kPairFlagBytes) != cudaSuccess) {
+      // (cleared on the stream that will use them: a stream may not wait for the default one)
+      if (cudaMalloc(&s.flags, kPairFlagBytes) != cudaSuccess || cudaMemsetAsync(s.flags, 0, kPairFlagBytes, ctx->stream) != cudaSuccess) {
         cudaGetLastError();
+        cudaFree(s.flags);
         cudaFree(s.slabs);
+        s.flags = nullptr;
         s.slabs = nullptr;
         return nullptr;
       }

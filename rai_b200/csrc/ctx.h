@@ -181,7 +181,7 @@ int gemm_pair_bf16(rb_ctx* ctx, const GemmArgs& a);   // gemm_pair.cu: M > 256, 
 // gemm_rows.cu: a bf16 product of at most eight rows with everything around it: rows are normalised first (norm: a kind, -1: no);
 // out = act(product + bias) + residual, act(product) * up product, or the plain sums as out_f
 struct RowsArgs {
-  const void *x = nullptr, *norm_w = nullptr, *norm_b = nullptr, *w = nullptr, *w2 = nullptr, *bias = nullptr, *residual = nullptr;
+  const void *x = nullptr, *norm_w = nullptr, *norm_b = nullptr, *w = nullptr, *w2 = nullptr, *bias = nullptr, *residual = nullptr, *act_params = nullptr;
   void* out = nullptr;
   float* out_f = nullptr;
   int64_t m = 0, n = 0, k = 0;
@@ -189,6 +189,7 @@ struct RowsArgs {
   float eps = 0.f;
 };
 bool gemm_rows_takes(int64_t m, int64_t k, bool norm);
+bool gemm_rows_pays(const rb_ctx* ctx, int64_t m, int64_t n, int64_t k);   // faster than split K on the kernel for more rows
 int gemm_rows(rb_ctx* ctx, const RowsArgs& a);
 constexpr int kMaxExperts = 256;
 int gemm_tc_grouped(rb_ctx* ctx, const GemmArgs& a);

@@ -33,7 +33,7 @@ constexpr int kRingBytes = kWarps * kTurns * kTurnSlices * 512;
 constexpr int kMostBytes = 212 * 1024;     // of shared memory (beside 8 KB of sums)
 
 struct RowsParams {
-  const bf16 *x, *w, *w2, *bias, *residual, *norm_w, *norm_b;
+  const bf16 *x, *w, *w2, *bias, *residual, *norm_w, *norm_b, *act_params;
   bf16* out;
   float* out_f;
   int m, n, k, act, norm, pitch, share;    // norm: an rb norm kind, or -1; pitch: bytes of a row of X; share: warps per tile
@@ -173,6 +173,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemm_rows_kernel(const RowsPar
   __syncthreads();
 
   // ---- tiles
+  const float2 ac = p.act == RB_ACT_XIELU ? xielu_consts(p.act_params) : make_float2(0.f, 0.f);
   const uint8_t* x_row = x_s + r * p.pitch + q * 16;
   const bool have = r < p.m;
   int slot = 0, flip = 0;
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemm_rows_kernel(const RowsPar
         v = act_apply(p.act, v) * v2;
       } else {
         if (p.bias) v += __bfloat162float(p.bias[col]);
-        v = act_apply(p.act, v) + extra[j];
+        v = act_apply(p.act, v, ac) + extra[j];
       }
       p.out[o] = __float2bfloat16_rn(v);
     }
@@ -260,11 +261,17 @@ bool gemm_rows_takes(int64_t m, int64_t k, bool norm) {
          (!norm || (k + 31) / 32 * 4 <= (int64_t)kNormPieces * 32 * (kWarps / m));
 }
 
+// Layered designs' products, by their size: of 8 x 3392 x 1024 and 8 x 1024 x 2048 (7 and 4 MB) a launch here takes about 4 us, against
+// 6 with split K and slabs for the consumer to sum; of 113 MB in four products 66 us against 58.
+bool gemm_rows_pays(const rb_ctx* ctx, int64_t m, int64_t n, int64_t k) {
+  return !ctx->debug_simple && !ctx->debug_simple_gemm && gemm_rows_takes(m, k, false) && n * k * 2 <= (20 << 20);
+}
+
 int gemm_rows(rb_ctx* ctx, const RowsArgs& a) {
   RB_REQUIRE(gemm_rows_takes(a.m, a.k, a.norm >= 0) && a.n > 0, "GEMM: %lld rows of %lld", (long long)a.m, (long long)a.k);
   RowsParams p{};
   p.x = (const bf16*)a.x; p.w = (const bf16*)a.w; p.w2 = (const bf16*)a.w2; p.bias = (const bf16*)a.bias;
-  p.residual = (const bf16*)a.residual; p.norm_w = (const bf16*)a.norm_w; p.norm_b = (const bf16*)a.norm_b;
+  p.residual = (const bf16*)a.residual; p.norm_w = (const bf16*)a.norm_w; p.norm_b = (const bf16*)a.norm_b; p.act_params = (const bf16*)a.act_params;
   p.out = (bf16*)a.out; p.out_f = a.out_f;
   p.m = (int)a.m; p.n = (int)a.n; p.k = (int)a.k; p.act = a.act; p.norm = a.norm; p.eps = a.eps;
   p.pitch = pitch_of(a.k);
@@ -280,7 +287,6 @@ int gemm_rows(rb_ctx* ctx, const RowsArgs& a) {
     RB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostBytes));
     set = true;
   }
-  ProfScope prof(ctx, RB_PROF_GEMM, 2.0 * ((a.w2 ? 2.0 : 1.0) * p.n * p.k + (double)p.m * p.k + (double)p.m * p.n), (a.w2 ? 4.0 : 2.0) * p.m * p.n * p.k);
   RB_CUDA(launch_kernel(kern, dim3((unsigned)grid), dim3(kWarps * 32), smem, ctx->stream, ctx->pdl, p));
   ctx->launches++;
   return RB_OK;

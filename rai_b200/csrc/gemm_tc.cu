@@ -762,6 +762,15 @@ int gemm_tc_bf16(rb_ctx* ctx, const GemmArgs& a) {
   RB_REQUIRE(a.k > 0 && (a.k % 8) == 0, "GEMM: K = %lld must be a positive multiple of 8", (long long)a.k);
   const bool gated = a.w2 != nullptr;
   RB_REQUIRE(!(gated && a.partials), "GEMM: split-K partials are not available for the gated form");
+  auto al16 = [](const void* v) { return (reinterpret_cast<uintptr_t>(v) & 15) == 0; };
+  if (!a.reduce && (!a.partials || a.n_split <= 1) && (a.act != RB_ACT_XIELU || (a.act_params && !gated)) &&
+      gemm_rows_pays(ctx, a.m, gated ? 2 * a.n : a.n, a.k) && al16(a.x) && al16(a.w) && al16(a.w2)) {
+    RowsArgs r;
+    r.x = a.x; r.w = a.w; r.w2 = a.w2; r.bias = a.bias; r.residual = a.residual; r.act = a.act; r.act_params = a.act_params;
+    r.m = a.m; r.n = a.n; r.k = a.k;
+    if (a.partials) r.out_f = (float*)a.out; else r.out = a.out;
+    return gemm_rows(ctx, r);
+  }
   Params p{};
   p.m = (int)a.m; p.n = (int)a.n; p.k = (int)a.k;
   p.num_kb = (int)((a.k + kBK - 1) / kBK);

@@ -59,6 +59,7 @@ int cache_dim(int dtype, int key_dim, int value_dim) {
 int slab_count(rb_model* m, int64_t rows, int64_t n, int64_t k) {
   if (m->cfg.dtype != RB_BF16 || rows > 256) return 0;
   const int fit = (int)std::min<size_t>(16, m->scratch_floats / ((size_t)rows * n));
+  if (gemm_rows_pays(m->ctx, rows, n, k)) return std::min(1, fit);
   return std::min(rb_linear_pick_splits(m->ctx, rows, n, k), fit);
 }
 
@@ -110,7 +111,7 @@ int mixer(rb_model* m, const MixLayer& w, int batch, int seq, const int32_t* new
 int mlp_up(rb_model* m, const MixLayer& w, int64_t rows, int act) {
   rb_ctx* ctx = m->ctx;
   const int64_t tiles = (w.mlp_k + 127) / 128;
-  if (!ctx->debug_simple && tiles * 4 < (int64_t)ctx->sm_count * 3) {
+  if (!ctx->debug_simple && tiles * 4 < (int64_t)ctx->sm_count * 3) {   // (a slab count of one: the epilogue does it)
     const int s = slab_count(m, rows, w.mlp_k, m->ld);
     if (s > 1) {
       RB_TRY(rb_linear_partials(ctx, m->h, w.up, m->scratch, rows, w.mlp_k, m->ld, s));

@@ -362,6 +362,10 @@ int few_rows_layer(rb_model* m, const LayerW& w, int l, int batch, int seq, int6
   o.out = down.out = m->h;
   o.residual = down.residual = m->h;
 
+  auto gemm_rows = [](rb_ctx* c, const RowsArgs& a) {
+    ProfScope prof(c, RB_PROF_GEMM, 2.0 * ((a.w2 ? 2.0 : 1.0) * a.n * a.k + (double)a.m * a.k + (double)a.m * a.n), (a.w2 ? 4.0 : 2.0) * a.m * a.n * a.k);
+    return rb::gemm_rows(c, a);
+  };
   RB_TRY(gemm_rows(ctx, qkv));
   if (phi2) RB_TRY(gemm_rows(ctx, up));   // the MLP reads the same normed rows as attention, before that adds to them (phi2.rs:293-299)
   if (seq == 1 && !pk) {

@@ -20,9 +20,9 @@
 // GATED computes act(X.Wg^T) * (X.Wu^T): a CTA's half of the W rows is 64 gate rows above the same 64 up rows, so one MMA
 // covers both and a column's gate and up sums lie 64 apart in the same lane.
 //
-// Measured against the one-SM kernel before it (M x N x K, us): 32768 x 3584 x 18944 3674 -> 3030, gated 32768 x 18944 x 3584
-// 8050 -> 6370 (1396 TFLOP/s of 1636 measured in bursts, 1373 sustained), 8192 x 9216 x 3072 444 -> 377, 4096 x 2560 x 10240 235 -> 175,
-// 1000 x 896 x 896 34 -> 18.
+// Measured against the one-SM kernel before it, a cool chip each time (M x N x K, us): 32768 x 3584 x 18944 3530 -> 2924, gated
+// 32768 x 18944 x 3584 7980 -> 6061 (1468 TFLOP/s of 1636 measured in bursts), 8192 x 9216 x 3072 350 -> 326, 4096 x 2560 x 10240 204 -> 159,
+// gated 3003 x 16384 x 2048 353 -> 290, 1000 x 896 x 896 25 -> 12.5.
 //
 // The epilogue turns rows into whole 128-byte pieces through shared memory, residual rows on their way in and results on
 // their way out; sums stay in float32 until the one rounding.

@@ -394,6 +394,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
               ok = seen != 0;
               *flag = 0;
             }
+            __syncwarp();   // what lane 0 acquired is there for the other lanes' loads (a shuffle orders no memory)
             ok = __shfl_sync(0xffffffffu, ok, 0);
             if (!ok) break;
             const float4* s = slab_of(h, place) + ch * (kCols / 4) * 32;

@@ -251,6 +251,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
         }
       }
       issued_count = (uint32_t)issued;
+      // the leader's commits of the last ring are counted in this CTA's shared memory, and nothing else waits for them
+      for (int i = 0; ok && i < kStages; ++i) {   // (a stage that was never filled: its barrier's phase before the first)
+        ok = ptx::mbar_wait(&empty_bar[stage], phase ^ 1u, &abort_flag, p.wait_cycles);
+        if (++stage == kStages) { stage = 0; phase ^= 1u; }
+      }
       if (!ok) { p.status[0] = (uint32_t)(-RB_ERR_TIMEOUT); p.status[1] = 0x6E11u; p.status[2] = blockIdx.x; }
     }
   } else if (warp == 1) {

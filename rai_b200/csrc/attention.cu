@@ -695,7 +695,7 @@ int launch_attention(rb_ctx* ctx, rb_kv_cache* c, AParams& p, int batch, int max
   }
   // Split the keys of a sequence over several blocks only when (sequence, KV head) pairs alone leave
   // the GPU under-filled: one long block per pair keeps its copy pipeline full and needs no merge.
-  const int splits = attention_decode_splits(ctx, batch, p.kv_heads, max_len, D);
+  const int splits = attention_decode_splits(ctx, batch, p.kv_heads, p.group, max_len, D);
   p.n_splits = splits;
   if (splits > 1) {
     RB_TRY(attention_reserve_scratch(ctx, (size_t)batch * p.q_heads * splits * (D + 2) * sizeof(float)));
@@ -736,7 +736,7 @@ static std::mutex g_static_attn_scratch_lock;
 
 template <int D>
 static int launch_attention_decode_static(rb_ctx* ctx, rb_kv_cache* c, AParams& p, int batch, int max_len, float* scratch) {
-  const int splits = attention_decode_splits(ctx, batch, p.kv_heads, max_len, D);
+  const int splits = attention_decode_splits(ctx, batch, p.kv_heads, p.group, max_len, D);
   p.n_splits = splits;
   if (splits > 1) {
     const size_t need = (size_t)batch * p.q_heads * splits * (D + 2);
@@ -758,26 +758,15 @@ static int launch_attention_decode_static(rb_ctx* ctx, rb_kv_cache* c, AParams& 
   return RB_OK;
 }
 
-int attention_decode_splits(rb_ctx* ctx, int batch, int kv_heads, int max_len, int head_dim) {
-  // One block per (sequence, KV head) keeps its copy pipeline full and needs no merge; splitting the
-  // keys only pays when those pairs under-fill the GPU.  Cost model in units of key tiles: a launch
-  // runs ceil(blocks / resident blocks) waves, each as long as one block's tiles plus a fixed start-up,
-  // and a split launch pays for handing its parts to whoever merges them, about six tiles (two query groups of seven heads of
-  // 64, us per step of 24 layers, split -> not: 2 tiles 744 -> 651, 5 tiles 747 -> 680, 10 tiles 782 -> 745; 8 tiles of 32 heads
-  // of 80 2053 -> 2161).
+// (RAI_B200_ATTN_SPLITS=n: n parts, or a tile each)
+int key_splits(const SplitCost& cost, int pairs, int max_len) {
   const int tiles = std::max(1, (max_len + kTile - 1) / kTile);
-  const int work = batch * kv_heads;
-  const int slots = (head_dim <= 128 ? 2 : 1) * ctx->sm_count;  // blocks resident at once (head size 256: one per SM)
-  int best = 1;
-  double best_cost = 1e30;
-  for (int s = 1; s <= std::min(tiles, 32); ++s) {
-    const int waves = (work * s + slots - 1) / slots;
-    const double cost = (double)waves * ((tiles + s - 1) / s + 2.0) + (s > 1 ? 6.0 : 0.0);
-    if (cost < best_cost - 1e-9) { best_cost = cost; best = s; }
-  }
   static const int forced = getenv("RAI_B200_ATTN_SPLITS") ? atoi(getenv("RAI_B200_ATTN_SPLITS")) : 0;
-  if (forced > 0) best = std::max(1, std::min(forced, tiles));
-  return best;
+  return forced > 0 ? std::max(1, std::min(forced, tiles)) : pick_key_splits(cost, pairs, tiles);
+}
+
+int attention_decode_splits(rb_ctx* ctx, int batch, int kv_heads, int group, int max_len, int head_dim) {
+  return key_splits(attention_split_cost(head_dim, group, ctx->sm_count), batch * kv_heads, max_len);
 }
 
 bool attention_mma_takes(const rb_kv_cache* c, int q_heads) {
@@ -808,7 +797,7 @@ int attention_mma_bf16(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, in
   p.wait_cycles = ctx->local_wait_cycles();
   RB_REQUIRE(p.group >= 1 && p.group <= 16 && q_heads % c->kv_heads == 0,
              "attention: %d query heads per KV head unsupported (1..16)", p.group);
-  // prefill with at least one 128-row query tile and head size 64 or 128: the tcgen05 kernel
+  // prefill with at least one 128-row query tile: the tcgen05 kernel
   if (ctx->attn_tc && attention_prefill_tc_supported(c, s_new, q_heads, q, out, ext != nullptr))
     return attention_prefill_tc(ctx, q, c, layer, batch, s_new, q_heads, scale, out, ext, pk);
   int max_len = 0;

@@ -678,7 +678,7 @@ int launch(rb_ctx* ctx, rb_kv_cache* c, Params p, int layer, int batch, int max_
   p.row_tiles = (whole + p.tile_rows - 1) / p.tile_rows;
   p.n_splits = 1;
   if (p.s_new == 1 && p.row_tiles <= (S::LATENT ? ::kLatentRowTiles : 1)) {
-    p.n_splits = attention_decode_splits(ctx, batch, p.row_tiles, max_len, 256);
+    p.n_splits = attention_joint_splits(ctx, c, p.q_heads, p.value_dim, batch, max_len);
     if (p.n_splits > kMaxSplits) p.n_splits = kMaxSplits;
     if (p.n_splits > 1) {
       const size_t parts = (size_t)batch * p.q_heads * p.n_splits;

@@ -28,10 +28,11 @@ int attention_latent_tc(rb_ctx* ctx, const joint::Params& p, rb_kv_cache* c, int
 
 }  // namespace
 
-int attention_joint_row_tiles(const rb_kv_cache* c, int q_heads) {
-  if (!c->shared()) return 1;
-  const int rows = c->head_dim > 512 ? 32 : 64;
-  return (q_heads + rows - 1) / rows;
+int attention_joint_splits(rb_ctx* ctx, const rb_kv_cache* c, int q_heads, int value_dim, int batch, int max_len) {
+  const int rows = !c->shared() ? q_heads : c->head_dim > 512 ? 32 : 64;   // of a block
+  const int row_tiles = (q_heads + rows - 1) / rows, nbk = c->head_dim / 64, nbv = (value_dim + 63) / 64;
+  const int tile_bytes = (c->shared() ? nbk : c->kv_heads * (nbk + nbv)) * 64 * 128;
+  return key_splits(joint_split_cost(tile_bytes, (q_heads + row_tiles - 1) / row_tiles * value_dim, ctx->sm_count), batch * row_tiles, max_len);
 }
 
 bool attention_joint_takes(const rb_kv_cache* c, const AttnExtra& x) {

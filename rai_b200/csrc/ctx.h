@@ -7,6 +7,7 @@
 #include <tuple>
 #include <vector>
 
+#include "attention_splits.h"
 #include "common.cuh"
 
 // What clusters that share a GEMM tile leave for one another (gemm_pair.cu): float32 sums and flags that the reader clears.
@@ -342,7 +343,8 @@ bool attention_can_fuse_rope(const rb_kv_cache* c, int q_heads, int rot, const v
 int attention_decode_fused_rope(rb_ctx* ctx, const void* qkv, const float* acc, int n_acc, const void* bias,
                                 const float* cos_t, const float* sin_t, int rot, rb_kv_cache* c, int layer, int batch,
                                 int q_heads, float scale, void* out);
-int attention_decode_splits(rb_ctx* ctx, int batch, int kv_heads, int max_len, int head_dim);
+int attention_decode_splits(rb_ctx* ctx, int batch, int kv_heads, int group, int max_len, int head_dim);
+int key_splits(const SplitCost& cost, int pairs, int max_len);
 // keys a single-token step may have to walk under a rolling window or in chunks, for the split decision above
 inline int attention_walk_len(int max_len, int window, int chunk = 0) {
   if (chunk > 0 && (window <= 0 || chunk < window)) window = chunk;
@@ -355,7 +357,7 @@ int attention_prefill_tc(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, 
                          void* out, const AttnExtra* ext = nullptr, const Packed* pk = nullptr);
 // attention_latent.cu, attention_talk.cu: attention with mixed heads or over latents, one block for all heads of its tokens
 bool attention_joint_takes(const rb_kv_cache* c, const AttnExtra& x);
-int attention_joint_row_tiles(const rb_kv_cache* c, int q_heads);   // blocks a single token's heads take
+int attention_joint_splits(rb_ctx* ctx, const rb_kv_cache* c, int q_heads, int value_dim, int batch, int max_len);   // of a single token's keys
 int attention_joint(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, int s_new, int q_heads, float scale, void* out,
                     const AttnExtra& x);
 // attention_mix_tc.cu: attention of prompts with mixed heads on tcgen05 (head sizes up to 128, up to 32 heads)

@@ -471,10 +471,10 @@ int rb::layered_decode_plan(rb_model* m, int batch) {
   uint32_t plan = 17;
   for (const MixLayer& w : m->mix)
     if (w.kv && w.c.block == RB_BLOCK_SANDWICH)
-      plan = plan * 31 + (uint32_t)attention_decode_splits(m->ctx, batch, attention_joint_row_tiles(w.kv, w.c.heads), max_len, 256);
+      plan = plan * 31 + (uint32_t)attention_joint_splits(m->ctx, w.kv, w.c.heads, w.c.mixer == RB_MIXER_LATENT ? w.kr_p : w.c.value_dim, batch, max_len);
     else if (w.kv)
-      plan = plan * 31 + (uint32_t)attention_decode_splits(m->ctx, batch, w.c.kv_heads, attention_walk_len(max_len, w.c.window, w.c.chunk),
-                                                           w.kv->head_dim);
+      plan = plan * 31 + (uint32_t)attention_decode_splits(m->ctx, batch, w.c.kv_heads, w.c.heads / w.c.kv_heads,
+                                                           attention_walk_len(max_len, w.c.window, w.c.chunk), w.kv->head_dim);
   return (int)(plan & 0x7fffffffu);
 }
 

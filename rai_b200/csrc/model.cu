@@ -1255,7 +1255,7 @@ int decode_plan(rb_model* m, int batch) {
   if (m->layered) return layered_decode_plan(m, batch);
   int max_len = 0;
   for (int b = 0; b < batch; ++b) max_len = std::max(max_len, m->cache->host_lens[b]);
-  return attention_decode_splits(m->ctx, batch, m->nkv_l, max_len, m->d);
+  return attention_decode_splits(m->ctx, batch, m->nkv_l, m->nq_l / m->nkv_l, max_len, m->d);
 }
 
 int decode_step_launches(rb_model* m, int batch) {

@@ -118,11 +118,18 @@ int32_t rb_set_wait_budget_us(rb_ctx* ctx, int64_t microseconds);
  * mbarrier nothing arrives on, waited for with the library's own helper; 1: the tensor-parallel exchange of a
  * two-member group whose second member, zeroed memory of this GPU, never raises its flag; 2: the same exchange
  * in its flag-inside-the-data form, whose second member's words never show the exchange number; 3: that form over
- * two hops, where one row waits for the other member's share and the other row for its finished sum), with the given
+ * two hops, where one row waits for the other member's share and the other row for its finished sum; 4: no
+ * kernel, but the flags that one may leave raised in a workspace of cut products, which rb_sync clears), with the given
  * budget.  The kernel returns when the budget runs out; RB_OK means the give-up was recorded as designed
  * (RB_ERR_TIMEOUT with the kernel's tag, outputs untouched), and the status word is clear again on return.
  * Nothing faults, traps or spins without bound.  No counterpart in the reference. */
 int32_t rb_selftest_wait_gives_up(rb_ctx* ctx, int32_t which, int64_t budget_us);
+/* Test hook: rb_linear (w2_dev NULL) or rb_gated_linear in bf16 on the kernel of prompt products with tiles of `tile_rows` (256 or
+ * 512) rows, cut along K as a model's products are if `cut` is not 0; rb_linear itself never cuts.  Allocates, synchronises and frees.
+ * RB_ERR_CUDA if the launch left its workspace unfit for the next one.  rows > 256 (gated: > 128).  No counterpart in the reference. */
+int32_t rb_selftest_pair_linear(rb_ctx* ctx, const void* x_dev, const void* w_dev, const void* w2_dev, const void* bias_dev,
+                                const void* residual_dev, void* out_dev, int64_t rows, int64_t n, int64_t k, int32_t act,
+                                int32_t tile_rows, int32_t cut);
 
 /* Device memory owned by the library (`TensorLike` storage, rai-core/src/tensor.rs:19-26). */
 int32_t rb_malloc(rb_ctx* ctx, size_t bytes, void** out_dev);

@@ -195,6 +195,7 @@ extern "C" {
     pub fn rb_sm_count(ctx: *mut rb_ctx) -> i32;
     pub fn rb_set_wait_budget_us(ctx: *mut rb_ctx, microseconds: i64) -> i32;
     pub fn rb_selftest_wait_gives_up(ctx: *mut rb_ctx, which: i32, budget_us: i64) -> i32;
+    pub fn rb_selftest_pair_linear(ctx: *mut rb_ctx, x_dev: *const c_void, w_dev: *const c_void, w2_dev: *const c_void, bias_dev: *const c_void, residual_dev: *const c_void, out_dev: *mut c_void, rows: i64, n: i64, k: i64, act: i32, tile_rows: i32, cut: i32) -> i32;
     pub fn rb_malloc(ctx: *mut rb_ctx, bytes: usize, out_dev: *mut *mut c_void) -> i32;
     pub fn rb_free(ctx: *mut rb_ctx, dev: *mut c_void) -> i32;
     pub fn rb_malloc_async(ctx: *mut rb_ctx, bytes: usize, out_dev: *mut *mut c_void) -> i32;

@@ -106,7 +106,6 @@ extern "C" int32_t rb_destroy(rb_ctx* ctx) {
   for (void* r : ctx->retired) cudaFree(r);
   if (ctx->gemm_scratch) cudaFree(ctx->gemm_scratch);
   if (ctx->gemm_tile_count) cudaFree(ctx->gemm_tile_count);
-  for (PairSpace& p : ctx->pair_space) { cudaFree(p.slabs); cudaFree(p.flags); }
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
   delete ctx;
   return RB_OK;
@@ -133,14 +132,15 @@ extern "C" int32_t rb_sync(rb_ctx* ctx) {
     RB_CUDA(cudaMemset(ctx->status_dev, 0, 4 * sizeof(uint32_t)));
     const int code = -(int)w[0];
     if (code == RB_ERR_TIMEOUT) {
-      // blocks that gave up returned before they were counted: re-arm the self-resetting arrival counters
+      // blocks that gave up returned before they were counted: re-arm the self-resetting arrival counters, once no stream
+      // has a launch under way that counts in them (every wait in those is bounded)
+      RB_CUDA(cudaDeviceSynchronize());
       for (rb_kv_cache* kc : ctx->caches)
         RB_CUDA(cudaMemset(kc->split_count, 0, kc->split_counters() * sizeof(uint32_t)));
       RB_CUDA(cudaMemset(ctx->argmax_best, 0, kArgmaxRows * sizeof(unsigned long long)));
       RB_CUDA(cudaMemset(ctx->argmax_count, 0, kArgmaxRows * sizeof(unsigned int)));
       RB_CUDA(cudaMemset(ctx->gemm_tile_count, 0, 2 * kGemmMaxReduceTiles * sizeof(uint32_t)));
-      for (PairSpace& p : ctx->pair_space)
-        if (p.flags) RB_CUDA(cudaMemset(p.flags, 0, kPairFlagBytes));
+      for (uint32_t* f : ctx->pair_flags) RB_CUDA(cudaMemset(f, 0, kPairFlagBytes));
       RB_CUDA(cudaStreamSynchronize(nullptr));  // the words are clear before any stream's next launch
     }
     return fail(code, "device-side check failed: code %d at 0x%x (detail %u, %u)", code, w[1], w[2], w[3]);

@@ -10,13 +10,13 @@
 #include "attention_splits.h"
 #include "common.cuh"
 
-// What clusters that share a GEMM tile leave for one another (gemm_pair.cu): float32 sums and flags that the reader clears.
-// One per stream, for the first kPairStreams streams that need one.
-constexpr int kPairStreams = 4, kPairClusters = 74;
+// What clusters that share a GEMM tile leave for one another (gemm_pair.cu): float32 sums and flags that the reader clears.  A
+// model owns one, as it owns its activations, and lends it to the products it issues (PairLoan): a model's calls follow one another,
+// whichever stream or graph they are on.  Nobody answers for that where rb_linear is called by itself; those products have none.
+constexpr int kPairClusters = 74;
 constexpr size_t kPairSlabBytes = (size_t)kPairClusters * 4 * 128 * 256 * sizeof(float);
 constexpr size_t kPairFlagBytes = (size_t)kPairClusters * 4 * 8 * sizeof(uint32_t);
 struct PairSpace {
-  cudaStream_t stream = nullptr;
   float* slabs = nullptr;
   uint32_t* flags = nullptr;
 };
@@ -38,7 +38,8 @@ struct rb_ctx {
   float* gemm_scratch = nullptr;   // float32 slabs of the GEMMs that reduce split-K inside the kernel; grow-only
   size_t gemm_scratch_bytes = 0;
   uint32_t* gemm_tile_count = nullptr;  // [2][kGemmMaxReduceTiles] arrival / done counters of those GEMMs, self-resetting
-  PairSpace pair_space[kPairStreams];
+  const PairSpace* pair_space = nullptr;    // lent for the call at hand; NULL: products are not cut
+  std::vector<uint32_t*> pair_flags;        // of every PairSpace there is, for rb_sync to clear
   long long wait_budget_cycles = 2000000000LL;  // give-up time of a device-side wait for ANOTHER GPU (rb_set_wait_budget_us)
   // Waits inside one kernel (operand rings, accumulators, sibling blocks) may begin before the kernel's predecessor
   // has finished, and that predecessor may itself be waiting for a peer: they get four times the budget, so that
@@ -178,7 +179,15 @@ struct GemmArgs {
   bool reduce = false;            // M <= 64: if K is split, sum the splits inside the kernel and apply the epilogue
 };
 int gemm_tc_bf16(rb_ctx* ctx, const GemmArgs& a);
-int gemm_pair_bf16(rb_ctx* ctx, const GemmArgs& a);   // gemm_pair.cu: M > 256, no partials
+// gemm_pair.cu: M > 256 (gated: > 128), no partials.  tile_rows: 0, or 256 or 512 to have that tile and whatever cut it allows
+int gemm_pair_bf16(rb_ctx* ctx, const GemmArgs& a, int tile_rows = 0);
+struct PairLoan {   // for the products issued in its scope
+  rb_ctx* ctx;
+  const PairSpace* before;
+  PairLoan(rb_ctx* c, const PairSpace& s) : ctx(c), before(c->pair_space) { c->pair_space = s.slabs ? &s : nullptr; }
+  ~PairLoan() { ctx->pair_space = before; }
+  PairLoan(const PairLoan&) = delete;
+};
 // gemm_rows.cu: a bf16 product of at most eight rows with everything around it: rows are normalised first (norm: a kind, -1: no);
 // out = act(product + bias) + residual, act(product) * up product, or the plain sums as out_f
 struct RowsArgs {

@@ -12,9 +12,9 @@
 // warp has 32 rows x 128 columns and gives the accumulator back once the last of them are in registers; with MT = 512 the
 // products of the first half run ahead while the second half is still drained.
 //
-// Persistent: 74 clusters stride over the tiles.  Where the tiles do not fill the last round, that round's tiles are cut along K
-// in equal shares for all clusters and done first: a cluster's share is the end of one tile and perhaps the start of the next.
-// Whoever has a tile's end finishes it, with the float32 sums that the others (all of them clusters before it, none of which
+// Persistent: 74 clusters stride over the tiles.  Where the tiles do not fill the last round and the caller has lent a workspace
+// (ctx.h), that round's tiles are cut along K in equal shares for all clusters and done first: a cluster's share is the end of one
+// tile and perhaps the start of the next.  Which tiles are cut, and so the order of their sums, depends on the sizes alone.  Whoever has a tile's end finishes it, with the float32 sums that the others (all of them clusters before it, none of which
 // waits for anyone, and each does the start of a tile first) left in global memory, added in a fixed order.
 //
 // GATED computes act(X.Wg^T) * (X.Wu^T): a CTA's half of the W rows is 64 gate rows above the same 64 up rows, so one MMA
@@ -508,35 +508,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant
   }
 }
 
-// The workspace of cut tiles that belongs to the context's current stream (launches on one stream follow one another; two
-// streams may overlap), or NULL: a stream beyond the first kPairStreams, or one that is being captured (a graph may be
-// replayed on any stream).
-PairSpace* pair_space(rb_ctx* ctx) {
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  for (PairSpace& s : ctx->pair_space) {
-    if (s.slabs && s.stream == ctx->stream) return &s;
-    if (!s.slabs) {
-      if (cudaMalloc(&s.slabs, kPairSlabBytes) != cudaSuccess) { cudaGetLastError(); s.slabs = nullptr; return nullptr; }
-      // (cleared on the stream that will use them: a stream may not wait for the default one)
-      if (cudaMalloc(&s.flags, kPairFlagBytes) != cudaSuccess || cudaMemsetAsync(s.flags, 0, kPairFlagBytes, ctx->stream) != cudaSuccess) {
-        cudaGetLastError();
-        cudaFree(s.flags);
-        cudaFree(s.slabs);
-        s.flags = nullptr;
-        s.slabs = nullptr;
-        return nullptr;
-      }
-      s.stream = ctx->stream;
-      return &s;
-    }
-  }
-  return nullptr;
-}
-
 int most_clusters(const rb_ctx* ctx) { return std::min(ctx->sm_count / 2, kPairClusters); }
 
 // How a product is shared out with tiles of mt rows, and what that costs in K blocks of a 256-row tile (about 0.25 us alone,
@@ -559,7 +530,7 @@ Split plan_split(const rb_ctx* ctx, int m, int n_out, int out_cols, int num_kb, 
   const int left = (int)(tiles % most);
   const int64_t rounds = tiles / most;
   double last = left > 0 ? num_kb : 0.0;
-  if (left > 0) {
+  if (left > 0 && ctx->pair_space) {
     const double move = 2.5, wait = (rounds > 0 ? 10.0 : 30.0) * 256 / mt;
     const double each = std::max(1.0, std::min((double)most / left, sqrt(num_kb / move)));   // clusters per cut tile
     const int shares = std::min(most, (int)(left * each));
@@ -592,15 +563,12 @@ int launch_pair(rb_ctx* ctx, const GemmArgs& a, PairParams& p, const Split& spli
   p.n_q = split.n_q;
   p.tiles = p.n_p * p.n_q;
   int clusters = std::min(p.tiles, most_clusters(ctx));
-  p.cut_tiles = p.cut_clusters = 0;
+  p.cut_tiles = split.cut;
+  p.cut_clusters = split.shares;
   if (split.shares > 0) {
-    if (PairSpace* s = pair_space(ctx)) {
-      p.cut_tiles = split.cut;
-      p.cut_clusters = split.shares;
-      p.slabs = s->slabs;
-      p.flags = s->flags;
-      clusters = std::max(clusters, split.shares);
-    }
+    p.slabs = ctx->pair_space->slabs;
+    p.flags = ctx->pair_space->flags;
+    clusters = std::max(clusters, split.shares);
   }
   RB_CUDA(launch_kernel(kern, dim3((unsigned)(2 * clusters)), dim3(kThreads), kSmemBytes, ctx->stream, ctx->pdl, tx, tw, tw2, p));
   ctx->launches++;
@@ -609,7 +577,7 @@ int launch_pair(rb_ctx* ctx, const GemmArgs& a, PairParams& p, const Split& spli
 
 }  // namespace
 
-int gemm_pair_bf16(rb_ctx* ctx, const GemmArgs& a) {
+int gemm_pair_bf16(rb_ctx* ctx, const GemmArgs& a, int tile_rows) {
   PairParams p{};
   p.m = (int)a.m;
   p.n = (int)a.n;
@@ -623,7 +591,8 @@ int gemm_pair_bf16(rb_ctx* ctx, const GemmArgs& a) {
   p.wait_cycles = ctx->local_wait_cycles();
   const int out_cols = a.w2 ? kBN / 2 : kBN;
   const Split narrow = plan_split(ctx, p.m, p.n, out_cols, p.num_kb, 256), wide = plan_split(ctx, p.m, p.n, out_cols, p.num_kb, 512);
-  if (wide.cost < narrow.cost) return a.w2 ? launch_pair<512, true>(ctx, a, p, wide) : launch_pair<512, false>(ctx, a, p, wide);
+  if (tile_rows == 512 || (tile_rows == 0 && wide.cost < narrow.cost))
+    return a.w2 ? launch_pair<512, true>(ctx, a, p, wide) : launch_pair<512, false>(ctx, a, p, wide);
   return a.w2 ? launch_pair<256, true>(ctx, a, p, narrow) : launch_pair<256, false>(ctx, a, p, narrow);
 }
 

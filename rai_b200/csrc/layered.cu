@@ -1019,6 +1019,7 @@ extern "C" int32_t rb_model_create_layers(rb_ctx* ctx, const rb_model_config* cf
 
   // ---- workspace.  Zeroed: what lies between a row's width and its pitch is multiplied by zero weights and must be finite.
   auto B = [&](size_t bytes, void** p) { if (st == RB_OK) st = dev_alloc(m, bytes, p, true); };
+  if (st == RB_OK) st = reserve_pair_space(m);
   const size_t MT = c.max_tokens, few = std::min<size_t>(MT, 256);
   B(MT * sizeof(uint32_t), (void**)&m->ids);
   B(MT * ld * sizeof(float), (void**)&m->stream);

@@ -144,6 +144,14 @@ int dev_alloc(rb_model* m, size_t bytes, void** out, bool zero) {
   return RB_OK;
 }
 
+int reserve_pair_space(rb_model* m) {
+  if (m->cfg.dtype != RB_BF16 || m->cfg.max_tokens <= 128) return RB_OK;   // (no product of a call is that large)
+  RB_TRY(dev_alloc(m, kPairSlabBytes, (void**)&m->pair_space.slabs, false));
+  RB_TRY(dev_alloc(m, kPairFlagBytes, (void**)&m->pair_space.flags, true));
+  m->ctx->pair_flags.push_back(m->pair_space.flags);
+  return RB_OK;
+}
+
 int weight_alloc(rb_model* m, int64_t elems, void** out) {
   m->param_bytes += elems * (int64_t)m->es;
   return dev_alloc(m, (size_t)elems * m->es, out, true);
@@ -407,6 +415,7 @@ int forward_impl(rb_model* m, const uint32_t* tokens, int batch, int seq, int po
 int forward_body(rb_model* m, const uint32_t* tokens, int batch, int seq, void* logits_out, const int32_t* rows_dev, int n_rows,
                  const int32_t* new_lens, const Packed* pk) {
   if (!rows_dev) n_rows = batch;
+  const PairLoan loan(m->ctx, m->pair_space);
   if (m->layered) {
     RB_TRY(layered_forward(m, tokens, batch, seq, new_lens));
     return finish_logits(m, batch, seq, logits_out, rows_dev, n_rows);
@@ -761,6 +770,7 @@ extern "C" int32_t rb_model_create(rb_ctx* ctx, const rb_model_config* cfg, rb_m
     st = attention_reserve_scratch(ctx, (size_t)c.max_batch * m->nq_l * 32 * (d + 2) * sizeof(float));
   if (st == RB_OK && c.dtype == RB_BF16)  // slabs of the GEMMs that reduce split-K in the kernel: 8 splits, 64 rows, two sets when gated
     st = gemm_reserve_scratch(ctx, (size_t)2 * 8 * 64 * std::max(m->inter_l, H) * sizeof(float));
+  if (st == RB_OK) st = reserve_pair_space(m);
   const size_t MT = c.max_tokens;
   W(MT * sizeof(uint32_t), (void**)&m->ids);
   W(MT * H * m->es, &m->h);
@@ -821,6 +831,8 @@ extern "C" int32_t rb_model_destroy(rb_model* m) {
   for (rb_kv_cache* v : m->views) rb_kv_cache_destroy(v);
   for (rb_kv_cache* v : m->prompt_kv) delete v;   // (their memory is the model's)
   if (m->cache) rb_kv_cache_destroy(m->cache);
+  std::vector<uint32_t*>& flags = m->ctx->pair_flags;
+  flags.erase(std::remove(flags.begin(), flags.end(), m->pair_space.flags), flags.end());
   for (void* p : m->owned) rb_free(m->ctx, p);
   delete m;
   return RB_OK;

@@ -101,6 +101,7 @@ struct rb_model {
   uint32_t* next_ids = nullptr;
   int32_t* last_rows = nullptr;           // the rows of a call whose logits are wanted [max_tokens]
   std::vector<int32_t> last_rows_host;    // outlives the asynchronous upload
+  PairSpace pair_space;      // of prompt products cut along K
   float* scratch = nullptr;  // split-K partials
   size_t scratch_floats = 0;
   void* comm = nullptr;
@@ -161,6 +162,7 @@ struct rb_model {
 namespace rb {
 int dev_alloc(rb_model* m, size_t bytes, void** out, bool zero);
 int weight_alloc(rb_model* m, int64_t elems, void** out);
+int reserve_pair_space(rb_model* m);
 void add_param(rb_model* m, const std::string& name, int64_t rows, int64_t cols, int rank, std::vector<Piece> pieces);
 // The launches between the token ids and the final residual stream of a layered design, and the logits of `n` of its rows
 // (row indices on the device, or NULL: the last row of each of the `n` sequences of `seq` rows).

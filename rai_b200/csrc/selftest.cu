@@ -1,6 +1,7 @@
 // Self-test of the give-up path of the bounded device-side waits (rb_selftest_wait_gives_up): kernels whose wait can
 // never be satisfied run with a short budget, and the host checks that they returned, that the status word
 // names them, and that nothing else was written.  Nothing here faults, traps or spins without bound.
+#include <algorithm>
 #include <vector>
 
 #include "ctx.h"
@@ -45,7 +46,7 @@ using namespace rb;
 
 extern "C" int32_t rb_selftest_wait_gives_up(rb_ctx* ctx, int32_t which, int64_t budget_us) {
   RB_REQUIRE(ctx, "rb_selftest_wait_gives_up: null context");
-  RB_REQUIRE(which >= 0 && which <= 3, "rb_selftest_wait_gives_up: unknown test %d", which);
+  RB_REQUIRE(which >= 0 && which <= 4, "rb_selftest_wait_gives_up: unknown test %d", which);
   RB_REQUIRE(budget_us >= 1 && budget_us <= 1000000, "rb_selftest_wait_gives_up: budget %lld us outside [1, 1 000 000]",
              (long long)budget_us);
   RB_TRY(rb_sync(ctx));  // start from a clear status word
@@ -64,6 +65,21 @@ extern "C" int32_t rb_selftest_wait_gives_up(rb_ctx* ctx, int32_t which, int64_t
     if (returned != 1u || w[0] != (uint32_t)(-RB_ERR_TIMEOUT) || w[1] != 0x5E1Fu)
       return fail(RB_ERR_CUDA, "wait self-test: expected a recorded give-up at 0x5E1F, got returned=%u status={%u, 0x%x}",
                   returned, w[0], w[1]);
+    return RB_OK;
+  }
+  if (which == 4) {
+    DevBuf flags;
+    std::vector<uint32_t> words(kPairFlagBytes / sizeof(uint32_t), 1u);
+    RB_CUDA(cudaMalloc(&flags.p, kPairFlagBytes));
+    RB_CUDA(cudaMemcpy(flags.p, words.data(), kPairFlagBytes, cudaMemcpyHostToDevice));
+    const uint32_t gave_up[4] = {(uint32_t)(-RB_ERR_TIMEOUT), 0x6E13u, 0u, 0u};
+    RB_CUDA(cudaMemcpy(ctx->status_dev, gave_up, sizeof(gave_up), cudaMemcpyHostToDevice));
+    ctx->pair_flags.push_back((uint32_t*)flags.p);
+    const int st = rb_sync(ctx);
+    ctx->pair_flags.pop_back();
+    RB_CUDA(cudaMemcpy(words.data(), flags.p, kPairFlagBytes, cudaMemcpyDeviceToHost));
+    const bool clear = std::all_of(words.begin(), words.end(), [](uint32_t v) { return v == 0u; });
+    if (st != RB_ERR_TIMEOUT || !clear) return fail(RB_ERR_CUDA, "re-arm self-test: rb_sync gave %d, flags %s", st, clear ? "clear" : "raised");
     return RB_OK;
   }
   // ---- the tensor-parallel exchange over a two-member group that lives entirely in this GPU's memory; this launch
@@ -144,5 +160,39 @@ extern "C" int32_t rb_selftest_wait_gives_up(rb_ctx* ctx, int32_t which, int64_t
   if (w[0] != 0u || !written)
     return fail(RB_ERR_CUDA, "exchange-wait self-test: the healthy call after the give-up failed (status %u, outputs %s)", w[0],
                 written ? "as expected" : "wrong");
+  return RB_OK;
+}
+
+extern "C" int32_t rb_selftest_pair_linear(rb_ctx* ctx, const void* x, const void* w, const void* w2, const void* bias, const void* residual,
+                                           void* out, int64_t rows, int64_t n, int64_t k, int32_t act, int32_t tile_rows, int32_t cut) {
+  RB_REQUIRE(ctx && x && w && out, "rb_selftest_pair_linear: null argument");
+  RB_REQUIRE(tile_rows == 256 || tile_rows == 512, "rb_selftest_pair_linear: tiles of %d rows", tile_rows);
+  RB_REQUIRE(rows > (w2 ? 128 : 256) && rows <= (1 << 20) && n > 0 && n <= (1 << 20) && k > 0 && k % 8 == 0, "rb_selftest_pair_linear: sizes");
+  RB_REQUIRE(act != RB_ACT_XIELU && !(w2 && (bias || residual)), "rb_selftest_pair_linear: not with these operands");
+  GemmArgs a;
+  a.x = x; a.w = w; a.w2 = w2; a.bias = bias; a.residual = residual; a.out = out;
+  a.m = rows; a.n = n; a.k = k; a.act = act;
+  DevBuf slabs, flags;
+  PairSpace space;
+  if (cut) {
+    RB_CUDA(cudaMalloc(&slabs.p, kPairSlabBytes));
+    RB_CUDA(cudaMalloc(&flags.p, kPairFlagBytes));
+    RB_CUDA(cudaMemsetAsync(slabs.p, 0xff, kPairSlabBytes, ctx->stream));   // (not numbers: what is read must have been written)
+    RB_CUDA(cudaMemsetAsync(flags.p, 0, kPairFlagBytes, ctx->stream));
+    space.slabs = (float*)slabs.p;
+    space.flags = (uint32_t*)flags.p;
+  }
+  int st;
+  {
+    const PairLoan loan(ctx, space);
+    st = gemm_pair_bf16(ctx, a, tile_rows);
+  }
+  RB_CUDA(cudaStreamSynchronize(ctx->stream));   // (before the workspace goes)
+  RB_TRY(st);
+  RB_TRY(rb_sync(ctx));
+  if (!cut) return RB_OK;
+  std::vector<uint32_t> words(kPairFlagBytes / sizeof(uint32_t));
+  RB_CUDA(cudaMemcpy(words.data(), flags.p, kPairFlagBytes, cudaMemcpyDeviceToHost));
+  if (std::any_of(words.begin(), words.end(), [](uint32_t v) { return v != 0u; })) return fail(RB_ERR_CUDA, "rb_selftest_pair_linear: a flag was left raised");
   return RB_OK;
 }

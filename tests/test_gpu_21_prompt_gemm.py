@@ -5,7 +5,8 @@ import ctypes
 import pytest
 import torch
 
-from rai_b200 import _lib
+from rai_b200 import _lib, configs, synth
+from rai_b200.models import Model
 
 pytestmark = pytest.mark.gpu
 P = lambda t: ctypes.c_void_p(t.data_ptr()) if t is not None else None  # noqa: E731
@@ -77,8 +78,8 @@ def test_infinities_and_nan_stay_in_their_rows(cuda):
     assert torch.equal(out[keep], clean[keep])
 
 
-def test_cut_tiles_on_several_streams_and_under_capture(cuda):
-    """Streams have workspaces of their own; a captured launch, and a stream too many, use whole tiles."""
+def test_same_bits_on_every_stream_and_under_capture(cuda):
+    """A product called by itself has no workspace that a stream or a graph could share with another."""
     x, w, _, _, _ = operands(300, 512, 8192, torch.bfloat16, 3)
     ref = linear_ref(x, w, None, None, _lib.ACT_NONE)
     streams, outs = [torch.cuda.Stream() for _ in range(2)], []
@@ -98,6 +99,56 @@ def test_cut_tiles_on_several_streams_and_under_capture(cuda):
     cuda.synchronize()
     for out in outs + [static]:
         assert float((out.double() - ref).abs().max()) <= bound(torch.bfloat16, ref, 8192)
+        assert torch.equal(out, outs[0])
+
+
+def test_a_row_has_the_same_bits_in_any_batch(cuda):
+    cuda.use_torch_stream()
+    x, w, w2, _, _ = operands(1300, 512, 8192, torch.bfloat16, 5)
+    whole = linear(cuda, x, w, None, None, _lib.ACT_NONE)
+    for m in (257, 300, 700):
+        assert torch.equal(linear(cuda, x[:m].contiguous(), w, None, None, _lib.ACT_NONE), whole[:m])
+    cuda.synchronize()
+
+
+def test_products_by_themselves_allocate_nothing(cuda):
+    """Every stream's first product, too: a host that owns the GPU's memory does not see it shrink."""
+    x, w, _, _, _ = operands(300, 512, 8192, torch.bfloat16, 6)
+    out = torch.empty(300, 512, dtype=torch.bfloat16, device="cuda")
+    streams = [torch.cuda.Stream() for _ in range(3)]
+
+    def product(s):
+        with torch.cuda.stream(s):
+            cuda.use_torch_stream()
+            _lib.call("rb_linear", cuda.ctx, P(x), P(w), None, None, P(out), 300, 512, 8192, _lib.ACT_NONE, _lib.BF16)
+        s.synchronize()
+
+    product(torch.cuda.default_stream())     # (the kernel's code is loaded)
+    free = torch.cuda.mem_get_info()[0]
+    for s in streams:
+        product(s)
+    left = torch.cuda.mem_get_info()[0]
+    cuda.use_torch_stream()
+    assert free - left < 8 << 20
+
+
+def test_a_model_on_any_stream_has_the_same_bits(cuda):
+    """A model's products are cut along K in a workspace of its own, whichever stream its calls come on."""
+    cfg = configs.get("qwen2-0.5b")
+    cfg.update(num_hidden_layers=2, vocab_size=512)
+    m = Model(cfg, _lib.BF16, cuda, 1, 320, 320)
+    m.update_params(synth.weights(cfg, 8))
+    ids = synth.prompt(cfg, 1, 300, 8)
+    outs = []
+    torch.cuda.synchronize()
+    for s in [torch.cuda.Stream() for _ in range(7)]:
+        with torch.cuda.stream(s):
+            m.clear_kv_cache()
+            outs.append(m.forward(ids, 0))
+        s.synchronize()
+    cuda.use_torch_stream()
+    assert all(torch.equal(o, outs[0]) for o in outs)
+    m.close()
 
 
 # rows: few (a dot product per row) and many (tiles of 16 to 128 rows); features around a tile; K cut in up to eight shares, not a

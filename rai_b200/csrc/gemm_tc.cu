@@ -13,7 +13,8 @@
 //
 // Operands are named by the TMEM axis they feed: the P operand's rows become TMEM lanes (128 per
 // tile), the Q operand's rows become TMEM columns (BN per tile).
-//   normal (SWAP = false): P = X, Q = W  — experts with many rows each (plain prefill-sized products: gemm_pair.cu).
+//   normal (SWAP = false): P = X, Q = W  — experts with many rows each, and short prompts without a residual (one_sm_pays; other
+//            prefill-sized products: gemm_pair.cu).
 //   swapped (SWAP = true):  P = W, Q = X  — decode-sized M (<= 256): the weight matrix, which is
 //            all of the HBM traffic, streams through the 128-row side at full tile efficiency while
 //            the few activation rows ride along as the narrow N side.  Two forms of split-K, both through
@@ -134,7 +135,6 @@ template <int BN, bool SWAP, bool GATED, int GROUP>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__ CUtensorMap tm_p2,
                const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_q2, const Params p) {
-  static_assert(SWAP || GROUP != 0, "plain products of many rows: gemm_pair.cu");
   constexpr bool kGather = GROUP != 0 && SWAP;  // rows by index
   static_assert(!kGather || BN <= 128, "one gather per lane");
   constexpr int kRowTile = SWAP ? BN : kBM;
@@ -244,13 +244,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
       // decode-sized GEMMs read every weight byte exactly once: evict-first keeps them from pushing
       // the activations and split-K partials out of L2
       const uint64_t stream_policy = ptx::policy_evict_first();
-      auto load_weights = [&](uint8_t* st, int stage, int kb, int pt) {
-        ptx::tma_load_2d_hint(st, &tm_p, &full_bar[stage], kb * kBK, pt * kBM, stream_policy);
-        if (C::kPTiles == 2)
-          ptx::tma_load_2d_hint(st + C::kPBytes, &tm_p2, &full_bar[stage], kb * kBK, pt * kBM, stream_policy);
+      auto load_weights = [&](uint8_t* st, int stage, int kb, int pt, int qt) {
+        if (SWAP) {
+          ptx::tma_load_2d_hint(st, &tm_p, &full_bar[stage], kb * kBK, pt * kBM, stream_policy);
+          if (C::kPTiles == 2)
+            ptx::tma_load_2d_hint(st + C::kPBytes, &tm_p2, &full_bar[stage], kb * kBK, pt * kBM, stream_policy);
+        } else {
+          uint8_t* qs = st + C::kPTiles * C::kPBytes;
+          ptx::tma_load_2d(qs, &tm_q, &full_bar[stage], kb * kBK, qt * BN);
+          if (C::kQTiles == 2) ptx::tma_load_2d(qs + C::kQBytes, &tm_q2, &full_bar[stage], kb * kBK, qt * BN);
+        }
       };
-      auto load_activations = [&](uint8_t* st, int stage, int kb, int qt) {
-        ptx::tma_load_2d(st + C::kPTiles * C::kPBytes, &tm_q, &full_bar[stage], kb * kBK, qt * BN);
+      auto load_activations = [&](uint8_t* st, int stage, int kb, int pt, int qt) {
+        if (SWAP) ptx::tma_load_2d(st + C::kPTiles * C::kPBytes, &tm_q, &full_bar[stage], kb * kBK, qt * BN);
+        else ptx::tma_load_2d(st, &tm_p, &full_bar[stage], kb * kBK, pt * kBM);
       };
       int n_pre = 0;
       for (int item = blockIdx.x; item < p.n_items && n_pre < n_stages; item += gridDim.x) {
@@ -259,7 +266,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
         const int kb0 = split * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
         for (int kb = kb0; kb < kb1 && n_pre < n_stages; ++kb, ++n_pre) {
           ptx::mbar_expect_tx(&full_bar[n_pre], C::kStageBytes);
-          load_weights(tiles + (size_t)n_pre * C::kStageBytes, n_pre, kb, pt);
+          load_weights(tiles + (size_t)n_pre * C::kStageBytes, n_pre, kb, pt, qt);
         }
       }
       pdl_wait();
@@ -276,9 +283,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
           if ((int)issued >= n_pre) {
             if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1u, &abort_flag, p.wait_cycles)) { ok = false; break; }
             ptx::mbar_expect_tx(&full_bar[stage], C::kStageBytes);
-            load_weights(st, stage, kb, pt);
+            load_weights(st, stage, kb, pt, qt);
           }
-          load_activations(st, stage, kb, qt);
+          load_activations(st, stage, kb, pt, qt);
           ++issued;
           if (++stage == n_stages) { stage = 0; phase ^= 1u; }
         }
@@ -462,10 +469,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_p, const __grid_constant__
         } else {
           const int gm = pt * kBM + lane_row;
           const int gn0 = qt * BN + c0;
+          if (GROUP == 0 && !GATED && p.bias) {
+#pragma unroll
+            for (int j8 = 0; j8 < CH; j8 += 8)
+              if (gn0 + j8 < p.n) {
+                float b8[8];
+                unpack8(*reinterpret_cast<const uint4*>(p.bias + gn0 + j8), b8);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j8 + j] += b8[j];
+              }
+          }
           if (GATED) act_inplace(p.act, g, ac);
           else if (p.act != RB_ACT_NONE) act_inplace(p.act, v, ac);
           if (gm < m_lim) {
-            const size_t o_row = GROUP == 1 ? row0 + gm : scatter[gm];  // (their columns come in eights)
+            const size_t o_row = GROUP == 0 ? gm : GROUP == 1 ? row0 + gm : scatter[gm];  // (columns come in eights)
 #pragma unroll
             for (int j8 = 0; j8 < CH; j8 += 8) {
               const int gn = gn0 + j8;
@@ -757,6 +774,24 @@ int gemm_reserve_scratch(rb_ctx* ctx, size_t bytes) {
   return RB_OK;
 }
 
+// Whether a product of many rows runs on single SMs, 128 x 256 (gated: 128 x 128) tiles, rather than on pairs.  A pair's launch costs about
+// 3 us more and has half as many, larger tiles, which fill few rounds badly; a single SM takes up to 1.3 times as long over a slice
+// of K once all of them are at work, and its epilogue waits for residual rows piece by piece.  us, pairs (whole tiles) -> single SMs:
+//   one round of tiles:  gated 129 x 4864 x 896 12.9 -> 9.5, plain 300 x 10240 x 2560 34.0 -> 20.9, gated 129 x 8192 x 3072 26.8 -> 26.6,
+//     but, with more slices, 600 x 2048 x 16384 91 -> 94 (cut along K 48)
+//   gated, few slices:   1400 x 4864 x 896 29 -> 22 (3 rounds against 4), 3000 x 2048 x 512 29 -> 22, but 1400 x 18944 x 3584 300 -> 467
+//   fewer rounds:        1400 x 10240 x 2560 with a bias 83 -> 66 (3 against 4)
+// Of 648 products of 129 to 3000 rows the rule makes none more than 3 % slower; their mean falls by 7 %.
+static bool one_sm_pays(const rb_ctx* ctx, const GemmArgs& a, int num_kb) {
+  if (a.residual || a.n % 8 != 0) return false;
+  const bool gated = a.w2 != nullptr;
+  const int64_t q = (a.n + (gated ? 127 : 255)) / (gated ? 128 : 256);
+  auto rounds = [&](int64_t rows, int64_t slots) { return ((a.m + rows - 1) / rows * q + slots - 1) / slots; };
+  const int64_t one = rounds(kBM, ctx->sm_count), pair = rounds(2 * kBM, ctx->sm_count / 2);
+  if (one == 1) return num_kb <= 56;
+  return gated ? num_kb <= 16 && one <= pair && one <= 4 : num_kb <= 56 && one < pair && one <= 3;
+}
+
 int gemm_tc_bf16(rb_ctx* ctx, const GemmArgs& a) {
   if (a.m == 0 || a.n == 0) return RB_OK;
   RB_REQUIRE(a.k > 0 && (a.k % 8) == 0, "GEMM: K = %lld must be a positive multiple of 8", (long long)a.k);
@@ -804,7 +839,10 @@ int gemm_tc_bf16(rb_ctx* ctx, const GemmArgs& a) {
     if (a.m <= 128) return launch<128, true, false>(ctx, a, p);
     return launch<256, true, false>(ctx, a, p);
   }
-  return gemm_pair_bf16(ctx, a);
+  if (!one_sm_pays(ctx, a, p.num_kb)) return gemm_pair_bf16(ctx, a);
+  p.p_rows = (int)a.m;
+  p.q_rows = (int)a.n;
+  return gated ? launch<128, false, true>(ctx, a, p) : launch<256, false, false>(ctx, a, p);
 }
 
 // The grouped form: a.m is the number of (row, choice) pairs.  a.x has a.m / a.top rows (a.up), or a.m compact rows (down, or

@@ -81,3 +81,29 @@ def test_qwen2_model_with_a_short_window(cuda, dtype, tol):
     assert util.logit_error(other, ref[0]) > 10 * tol
     m.close()
     m2.close()
+
+
+@pytest.mark.parametrize("dtype,tol", [(_lib.F32, 1e-4), (_lib.BF16, 2e-2)])
+def test_ragged_prompts_with_a_short_window(cuda, dtype, tol):
+    """Rows without their padding, in two calls: the window counts a sequence's own tokens of the call at hand."""
+    cfg = dict(configs.get("tiny-qwen2"), sliding_window=24)
+    w = synth.weights(cfg, 6)
+    oracle, g = util.build_oracle(cfg, w), np.random.default_rng(6)
+    parts = [[g.integers(0, cfg["vocab_size"], size=n) for n in lens] for lens in ([70, 5, 130, 33], [30, 64, 1, 27])]
+    m, got = Model(cfg, dtype, cuda, 4, 256, 4 * 130), []
+    m.update_params(w)
+    for part in parts:
+        lens = [len(p) for p in part]
+        ids = np.full((4, max(lens)), 3, dtype=np.int32)
+        for i, p in enumerate(part):
+            ids[i, :len(p)] = p
+        got.append(m.forward_rows(ids, lens, [i * max(lens) + n - 1 for i, n in enumerate(lens)]).float().cpu())
+    for i in range(4):
+        oracle.clear_kv_cache()
+        pos = 0
+        for part, logits in zip(parts, got):
+            want = oracle.forward(torch.from_numpy(part[i].astype(np.int64)).reshape(1, -1), pos).reshape(-1)
+            err = util.logit_error(logits[i], want) if dtype == _lib.BF16 else util.rel_error(logits[i], want)
+            assert err <= tol, f"sequence {i} at {pos}: error {err:.2e}"
+            pos += len(part[i])
+    m.close()

@@ -446,3 +446,15 @@ def test_heads_of_a_prompt(cuda, dtype, H, d, rd, turning, interleaved, kr, e, b
             assert (kk[:, d + rd:] == 0).all() and (vv[:, e:] == 0).all()
     prompt.close()
     cache.close()
+
+
+@pytest.mark.parametrize("B,T", [(1, 64), (1, 65), (1, 128), (1, 200), (1, 449), (5, 320), (5, 577), (9, 257), (80, 129)])
+def test_short_contexts_of_single_tokens(cuda, B, T):
+    """Lengths of one to ten tiles, whose keys one to ten blocks share depending on what a tile takes and how many sequences there are."""
+    H = 32 if B < 10 else 8
+    got, (q, k, v, talk) = talking_case(cuda, _lib.BF16, H, 8, 128, 128, T - 1, 1, B=B)
+    seqs = sorted({0, B // 2, B - 1})
+    want = np.stack([ref.attention(q[b, T - 1:], k[b], v[b], 0.2, None, talk, T - 1) for b in seqs])
+    assert rms_err(got[seqs], want) < TOL[_lib.BF16]
+    got, want = latent_case(cuda, _lib.BF16, 32, 512, 64, T - 1, 1, B=min(B, 9))
+    assert rms_err(got, want) < TOL[_lib.BF16]

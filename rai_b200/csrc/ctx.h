@@ -191,7 +191,7 @@ struct PairLoan {   // for the products issued in its scope
 // gemm_rows.cu: a bf16 product of at most eight rows with everything around it: rows are normalised first (norm: a kind, -1: no);
 // out = act(product + bias) + residual, act(product) * up product, or the plain sums as out_f
 struct RowsArgs {
-  const void *x = nullptr, *norm_w = nullptr, *norm_b = nullptr, *w = nullptr, *w2 = nullptr, *bias = nullptr, *residual = nullptr, *act_params = nullptr;
+  const void *x = nullptr, *norm_w = nullptr, *norm_b = nullptr, *w = nullptr, *w2 = nullptr, *bias = nullptr, *residual = nullptr;
   void* out = nullptr;
   float* out_f = nullptr;
   int64_t m = 0, n = 0, k = 0;

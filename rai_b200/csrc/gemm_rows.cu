@@ -27,13 +27,15 @@ using bf16 = __nv_bfloat16;
 namespace {
 
 constexpr int kWarps = 8;
-constexpr int kNormPieces = 12;            // 16-byte pieces of a row that a lane normalises at most
+// 16-byte pieces of a row that a lane normalises at most.  With 12 (a row's warps shared out among eight rows of more than 1024) a layer
+// was slower than on the kernels for more rows: 16 layers of 1536 x 6144, eight rows 764 -> 826 us, of 2048 x 5000 838 -> 977.
+constexpr int kNormPieces = 4;
 constexpr int kTurns = 3, kTurnSlices = 8; // a warp's ring: turns of eight slices (gated: four of gate and four of up)
 constexpr int kRingBytes = kWarps * kTurns * kTurnSlices * 512;
 constexpr int kMostBytes = 212 * 1024;     // of shared memory (beside 8 KB of sums)
 
 struct RowsParams {
-  const bf16 *x, *w, *w2, *bias, *residual, *norm_w, *norm_b, *act_params;
+  const bf16 *x, *w, *w2, *bias, *residual, *norm_w, *norm_b;
   bf16* out;
   float* out_f;
   int m, n, k, act, norm, pitch, share;    // norm: an rb norm kind, or -1; pitch: bytes of a row of X; share: warps per tile
@@ -54,8 +56,7 @@ __device__ __forceinline__ void mma_rows(float (&c)[4], uint32_t a0, uint32_t a2
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
 }
 
-// NP: 16-byte pieces of a row per lane, where rows are normalised
-template <bool GATED, int NP>
+template <bool GATED>
 __global__ void __launch_bounds__(kWarps * 32, 2) gemm_rows_kernel(const RowsParams p) {
   constexpr int G = GATED ? 2 : 1, U = kTurnSlices / G;   // slices per turn
   extern __shared__ __align__(128) uint8_t smem[];
@@ -109,14 +110,14 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemm_rows_kernel(const RowsPar
   } else {
     const int per_row = kWarps / p.m, row = warp / per_row, at = (warp % per_row) * 32 + lane, stride = per_row * 32;
     const bool work = row < p.m;
-    uint4 v[NP];
+    uint4 v[kNormPieces];
     float s = 0.f;
     const float inv_sqrt_h = 1.0f / sqrtf((float)p.k);
 #pragma unroll
-    for (int i = 0; i < NP; ++i)
+    for (int i = 0; i < kNormPieces; ++i)
       if (work && at + i * stride < pieces) v[i] = *reinterpret_cast<const uint4*>(p.x + (size_t)row * p.k + (at + i * stride) * 8);
 #pragma unroll
-    for (int i = 0; i < NP; ++i)
+    for (int i = 0; i < kNormPieces; ++i)
       if (work && at + i * stride < pieces) {
         float t[8];
         load8(reinterpret_cast<const bf16*>(&v[i]), t);
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemm_rows_kernel(const RowsPar
       mean = s / (float)p.k;
       float d2 = 0.f;
 #pragma unroll
-      for (int i = 0; i < NP; ++i)
+      for (int i = 0; i < kNormPieces; ++i)
         if (work && at + i * stride < pieces) {
           float t[8];
           load8(reinterpret_cast<const bf16*>(&v[i]), t);
@@ -153,7 +154,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemm_rows_kernel(const RowsPar
       scale = 1.0f / sqrtf((p.norm == RB_NORM_RMS ? s : s / (float)p.k) + p.eps);
     }
 #pragma unroll
-    for (int i = 0; i < NP; ++i) {
+    for (int i = 0; i < kNormPieces; ++i) {
       const int c = at + i * stride;
       if (!work || c >= padded) continue;
       float y[8] = {};
@@ -173,7 +174,6 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemm_rows_kernel(const RowsPar
   __syncthreads();
 
   // ---- tiles
-  const float2 ac = p.act == RB_ACT_XIELU ? xielu_consts(p.act_params) : make_float2(0.f, 0.f);
   const uint8_t* x_row = x_s + r * p.pitch + q * 16;
   const bool have = r < p.m;
   int slot = 0, flip = 0;
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemm_rows_kernel(const RowsPar
         v = act_apply(p.act, v) * v2;
       } else {
         if (p.bias) v += __bfloat162float(p.bias[col]);
-        v = act_apply(p.act, v, ac) + extra[j];
+        v = act_apply(p.act, v) + extra[j];
       }
       p.out[o] = __float2bfloat16_rn(v);
     }
@@ -271,18 +271,16 @@ int gemm_rows(rb_ctx* ctx, const RowsArgs& a) {
   RB_REQUIRE(gemm_rows_takes(a.m, a.k, a.norm >= 0) && a.n > 0, "GEMM: %lld rows of %lld", (long long)a.m, (long long)a.k);
   RowsParams p{};
   p.x = (const bf16*)a.x; p.w = (const bf16*)a.w; p.w2 = (const bf16*)a.w2; p.bias = (const bf16*)a.bias;
-  p.residual = (const bf16*)a.residual; p.norm_w = (const bf16*)a.norm_w; p.norm_b = (const bf16*)a.norm_b; p.act_params = (const bf16*)a.act_params;
+  p.residual = (const bf16*)a.residual; p.norm_w = (const bf16*)a.norm_w; p.norm_b = (const bf16*)a.norm_b;
   p.out = (bf16*)a.out; p.out_f = a.out_f;
   p.m = (int)a.m; p.n = (int)a.n; p.k = (int)a.k; p.act = a.act; p.norm = a.norm; p.eps = a.eps;
   p.pitch = pitch_of(a.k);
   const int tiles = (p.n + 7) / 8, grid = std::min(tiles, ctx->sm_count), each = (tiles + grid - 1) / grid;
   p.share = each >= 5 ? 1 : each >= 3 ? 2 : each == 2 ? 4 : 8;   // all of an SM's tiles at once, up to eight
   const size_t smem = (size_t)kRingBytes + p.m * p.pitch;
-  const bool short_rows = a.norm < 0 || (a.k + 31) / 32 * 4 <= 4 * 32 * (kWarps / a.m);
-  auto kern = a.w2 ? (short_rows ? gemm_rows_kernel<true, 4> : gemm_rows_kernel<true, kNormPieces>)
-                   : (short_rows ? gemm_rows_kernel<false, 4> : gemm_rows_kernel<false, kNormPieces>);
-  static bool attr_set[4][64] = {};  // the attribute belongs to the (kernel, device) pair
-  bool& set = attr_set[(a.w2 ? 2 : 0) + (short_rows ? 1 : 0)][ctx->device & 63];
+  auto kern = a.w2 ? gemm_rows_kernel<true> : gemm_rows_kernel<false>;
+  static bool attr_set[2][64] = {};  // the attribute belongs to the (kernel, device) pair
+  bool& set = attr_set[a.w2 ? 1 : 0][ctx->device & 63];
   if (!set) {
     RB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostBytes));
     set = true;

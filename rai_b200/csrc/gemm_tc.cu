@@ -15,7 +15,7 @@
 // tile), the Q operand's rows become TMEM columns (BN per tile).
 //   normal (SWAP = false): P = X, Q = W  — experts with many rows each, and short prompts without a residual (one_sm_pays; other
 //            prefill-sized products: gemm_pair.cu).
-//   swapped (SWAP = true):  P = W, Q = X  — decode-sized M (<= 256): the weight matrix, which is
+//   swapped (SWAP = true):  P = W, Q = X  — decode-sized M (<= 256, gated <= 128): the weight matrix, which is
 //            all of the HBM traffic, streams through the 128-row side at full tile efficiency while
 //            the few activation rows ride along as the narrow N side.  Two forms of split-K, both through
 //            float32 slabs in global memory (they stay in L2): `partials` leaves the slabs to the consumer
@@ -798,12 +798,10 @@ int gemm_tc_bf16(rb_ctx* ctx, const GemmArgs& a) {
   const bool gated = a.w2 != nullptr;
   RB_REQUIRE(!(gated && a.partials), "GEMM: split-K partials are not available for the gated form");
   auto al16 = [](const void* v) { return (reinterpret_cast<uintptr_t>(v) & 15) == 0; };
-  if (!a.reduce && (!a.partials || a.n_split <= 1) && (a.act != RB_ACT_XIELU || (a.act_params && !gated)) &&
-      gemm_rows_pays(ctx, a.m, gated ? 2 * a.n : a.n, a.k) && al16(a.x) && al16(a.w) && al16(a.w2)) {
+  if (a.partials && a.n_split <= 1 && gemm_rows_pays(ctx, a.m, a.n, a.k) && al16(a.x) && al16(a.w)) {
     RowsArgs r;
-    r.x = a.x; r.w = a.w; r.w2 = a.w2; r.bias = a.bias; r.residual = a.residual; r.act = a.act; r.act_params = a.act_params;
-    r.m = a.m; r.n = a.n; r.k = a.k;
-    if (a.partials) r.out_f = (float*)a.out; else r.out = a.out;
+    r.x = a.x; r.w = a.w; r.m = a.m; r.n = a.n; r.k = a.k;
+    r.out_f = (float*)a.out;
     return gemm_rows(ctx, r);
   }
   Params p{};

@@ -341,9 +341,10 @@ int mlp_up(rb_model* m, const LayerW& w, int64_t rows) {
 // Whether a layer of so few rows takes the kernels that fold norms and residual sums into the products.
 bool few_rows(const rb_model* m, int64_t rows) {
   const rb_model_config& c = m->cfg;
-  // Worth it where a layer's launches, not its bytes, are most of its time.  us per step, with the kernels for more rows -> these:
-  // 30 MB of weights a layer 1036 -> 651 (one row), 1058 -> 850 (eight); 157 MB 2035 -> 1959, 2212 -> 2206; 226 MB 2217 -> 2130 but,
-  // with four rows, 2821 -> 3083; 466 MB 3062 -> 3483.
+  // Worth it where a layer's launches, not its bytes, are most of its time: up to 96 MB of weights every number of rows gains.  us per
+  // step at 128 keys, with the kernels for more rows -> these, one / two / four rows: 28 MB a layer (24 of them) 991 -> 661, 989 -> 663,
+  // 993 -> 709, eight rows 1003 -> 772; 91 MB (16) 810 -> 724, 831 -> 729, 833 -> 702; 150 MB (32) 1947 -> 1705, 1966 -> 1900; 216 MB (32)
+  // 2134 -> 2176, 2161 -> 2058.  (Eight rows of more than 1024 and four of more than 2048 are not taken: kNormPieces.)
   const int64_t layer_weights = (int64_t)c.hidden_size * (m->nqkv_l + (int64_t)m->nq_l * m->d + (c.arch == RB_ARCH_PHI2 ? 2 : 3) * (int64_t)m->inter_l);
   if (layer_weights * 2 > (96 << 20)) return false;
   return c.dtype == RB_BF16 && c.tp_size == 1 && !m->ctx->debug_simple && !m->ctx->debug_simple_gemm && c.hidden_act != RB_ACT_XIELU &&
@@ -1091,10 +1092,11 @@ extern "C" int32_t rb_model_finished(rb_model* m, int32_t batch, uint8_t* flags_
   return RB_OK;
 }
 
-// The general step: sequence b feeds lens[b] (0..seq, NULL = seq) of the tokens in its row, followed by padding.  The
-// rectangle runs as usual (under the causal mask a pad can only influence later pads, and recurrent states stop at the
-// last token), logits come from the rows asked for, and the cache keeps lens[b] more tokens of sequence b: the pads'
-// K/V rows lie beyond that length, are never read, and are overwritten by the tokens fed next.
+// The general step: sequence b feeds lens[b] (0..seq, NULL = seq) of the tokens in its row, followed by padding.  The tokens alone
+// are packed into the rows of the call, and only they reach the cache.  Layered designs, and a call that wants the logits of
+// a padding row, run the whole rectangle instead: under the causal mask a pad can only influence later pads, recurrent states stop
+// at the last token, and the pads' K/V rows lie beyond the lengths that the cache keeps, are never read, and are overwritten
+// by the tokens fed next.
 // pos >= 0 must be every sequence's cached length; pos < 0 continues each at its own.
 static int forward_rows(rb_model* m, const uint32_t* tokens, int batch, int seq, int pos, const int32_t* lens, const int32_t* rows,
                         int n_rows, void* logits_out) {

@@ -78,15 +78,18 @@ __global__ void __launch_bounds__(256) rope_rows_kernel(const bf16* __restrict__
   }
 }
 
-constexpr int64_t kManyRows = 1024;   // several rows for every SM; below, a block per row starts more loads at once
+// Several rows for every SM, and rows wide enough that a block has work for more than its smallest 64 threads.  us, one item per thread -> this: 1024 rows
+// of 4608 columns 6.0 -> 5.2, of 2560 (one key head of 256) 5.9 -> 5.3; 16384 of 3072 56 -> 50, of 2560 (heads of 128) 50 -> 49, but of 1152
+// (qwen2-0.5b) 22 -> 38, of 2048 37 -> 48; 256 to 768 rows within 0.3 of one another but for heads of 80 and 96, where 512 gain already.
+constexpr int64_t kManyRows = 1024, kWideRow = 2560;
 
 }  // namespace
 
 // The caller has checked that rows are made of aligned 16-byte pieces.  false: its own kernel takes the call.
 bool rope_prompt(rb_ctx* ctx, const void* qkv, const float* cos_t, const float* sin_t, int rot, int rows, int s_new, int q_heads, rb_kv_cache* c,
                  void* k, void* v, void* q_out, const Packed* pk, cudaError_t* status) {
-  if (rows < kManyRows) return false;
   const int d = c->head_dim, rot_heads = q_heads + c->kv_heads;
+  if (rows < kManyRows || (rot_heads + c->kv_heads) * d < kWideRow) return false;
   const int work = std::max(rot / 16 * ((rot_heads + 3) / 4), (rot_heads * ((d - rot) / 8) + c->kv_heads * (d / 8) + 3) / 4);
   const int threads = std::max(64, std::min(256, (work + 31) / 32 * 32));
   *status = launch_kernel(rope_rows_kernel, dim3((unsigned)rows), dim3((unsigned)threads), 0, ctx->stream, ctx->pdl, (const bf16*)qkv, cos_t, sin_t,

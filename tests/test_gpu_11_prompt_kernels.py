@@ -12,7 +12,9 @@ P = lambda t: ctypes.c_void_p(t.data_ptr()) if t is not None else None  # noqa: 
 
 
 @pytest.mark.parametrize("nq,nkv,d,rot", [(4, 2, 64, 64), (3, 3, 80, 32), (2, 2, 96, 96), (7, 1, 128, 128), (8, 1, 256, 256), (5, 2, 64, 16),
-                                          (2, 1, 128, 0)])
+                                          (2, 1, 128, 0),
+                                          # rows as wide as the kernel for many of them wants, or wider
+                                          (28, 6, 64, 64), (30, 5, 64, 16), (16, 8, 80, 32), (24, 2, 96, 96), (21, 3, 128, 128), (18, 1, 128, 0)])
 def test_head_split_of_many_rows(cuda, nq, nkv, d, rot):
     """1200 rows at once, and in two calls of 600: the same bits in q and in the cache."""
     cuda.use_torch_stream()

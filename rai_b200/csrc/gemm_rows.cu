@@ -263,12 +263,12 @@ bool gemm_rows_takes(int64_t m, int64_t k, bool norm) {
 
 // Layered designs' products, by their size.  With the norm that reads it, alone in a chain of its like, a product of 2 MB takes 4.5 us
 // against 6.0 with split K and slabs for the consumer to sum, of 8 MB 5.2 against 6.5, of 20 MB 8.9 against 9.6, of 36 MB 15.3
-// against 14.3 (one row).  Between larger products that split K, one of few rows and many features either way costs more than that:
-// steps of malasun-2k (2048 x 2048, 8 MB) 618 -> 632 us with one row, 632 -> 644 with four, of votapel-2k 824 -> 852, while eight rows
-// gain (657 -> 641); with at most 1024 features on one side steps of the 1k designs are between 3 % longer and 5 % shorter, mostly shorter.
+// against 14.3 (one row).  Between larger products that split K, one of one to three rows and many features either way costs more than
+// that: a step of malasun-2k (2048 x 2048, 8 MB) with one row 618 -> 632 us at 128 keys, 641 -> 667 at 1500, of votapel-2k 824 -> 852.  From
+// four rows on it gains: malasun-2k, six rows at 1500 keys, 691 -> 673, fizadra-2k, four rows, 915 -> 893, kufulix-2k 973 -> 948.
 bool gemm_rows_pays(const rb_ctx* ctx, int64_t m, int64_t n, int64_t k) {
   return !ctx->debug_simple && !ctx->debug_simple_gemm && gemm_rows_takes(m, k, false) && n * k * 2 <= (20 << 20) &&
-         (m >= 7 || std::min(n, k) <= 1024);
+         (m >= 4 || std::min(n, k) <= 1024);
 }
 
 int gemm_rows(rb_ctx* ctx, const RowsArgs& a) {

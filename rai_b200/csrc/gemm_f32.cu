@@ -1,8 +1,8 @@
 // float32 Linear (the float32 models' rb_linear and rb_gated_linear) on CUDA cores: every product and sum is a float32 FMA.
 //
 // gemv_f32_kernel   M <= 8 rows (single-token steps): bound by the weight stream.  A feature's weight row is shared out among
-//                   1 to 8 warps, so that narrow layers, too, put enough warps on the GPU, and a lane requests all of its next
-//                   512 to 1024 bytes before it multiplies any of them.
+//                   1 to 8 warps, so that narrow layers, too, put enough warps on the GPU, and a lane requests 64 to 128 bytes of
+//                   the row (a warp 2 to 4 KB) before it multiplies any of them.
 // gemm_f32_kernel   more rows (prompts): bound by the FMA pipe.  Tiles of 16 TM rows x 64 features, TM chosen so that few rows
 //                   are padding; where the tiles alone do not fill the GPU, K is cut among the blocks of a cluster, which add
 //                   their sums through distributed shared memory in the order of K.

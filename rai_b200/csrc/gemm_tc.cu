@@ -782,12 +782,17 @@ int gemm_reserve_scratch(rb_ctx* ctx, size_t bytes) {
 //   gated, few slices:   1400 x 4864 x 896 29 -> 22 (3 rounds against 4), 3000 x 2048 x 512 29 -> 22, but 1400 x 18944 x 3584 300 -> 467
 //   fewer rounds:        1400 x 10240 x 2560 with a bias 83 -> 66 (3 against 4)
 // Of 648 products of 129 to 3000 rows the rule makes none more than 3 % slower; their mean falls by 7 %.
+// Without a workspace a pair's last round is not cut along K, and single SMs win at any K where all their tiles are at work at once, and
+// where two rounds of them stand against three or more of pairs: gated 300 x 5120 x 5120 100 -> 54, 513 x 3584 x 18944 200 -> 129, plain 300 x 12288 x 4096
+// 84 -> 49 (of 480 such products of 129 to 3000 rows 109 change sides, by 8 % in the mean and never for the worse by more than 4 %); three
+// rounds against four are not enough: gated 300 x 18944 x 3584 118 -> 133.
 static bool one_sm_pays(const rb_ctx* ctx, const GemmArgs& a, int num_kb) {
   if (a.residual || a.n % 8 != 0) return false;
   const bool gated = a.w2 != nullptr;
   const int64_t q = (a.n + (gated ? 127 : 255)) / (gated ? 128 : 256);
   auto rounds = [&](int64_t rows, int64_t slots) { return ((a.m + rows - 1) / rows * q + slots - 1) / slots; };
   const int64_t one = rounds(kBM, ctx->sm_count), pair = rounds(2 * kBM, ctx->sm_count / 2);
+  if (!ctx->pair_space && (one == 1 || (one == 2 && pair > 2))) return true;
   if (one == 1) return num_kb <= 56;
   return gated ? num_kb <= 16 && one <= pair && one <= 4 : num_kb <= 56 && one < pair && one <= 3;
 }

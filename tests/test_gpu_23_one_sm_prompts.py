@@ -56,3 +56,14 @@ def test_infinities_and_nan_stay_in_their_rows(cuda):
     assert torch.isnan(out[299]).all() and not torch.isfinite(out[130]).any()
     keep = [i for i in range(300) if i not in (130, 299)]
     assert torch.equal(out[keep], clean[keep])
+
+
+# rb_linear by itself has no workspace to be cut in: one round of tiles at any K, two where pairs need three
+@pytest.mark.parametrize("m,n,k", [(300, 520, 8200), (511, 3584, 4096), (513, 14336, 3592)])
+def test_linear_of_many_slices(cuda, m, n, k):
+    test_linear(cuda, m, n, k)
+
+
+@pytest.mark.parametrize("m,n,k", [(257, 264, 8200), (129, 4096, 4096), (257, 10240, 1032)])
+def test_gated_linear_of_many_slices(cuda, m, n, k):
+    test_gated_linear(cuda, m, n, k)

@@ -265,10 +265,17 @@ int dispatch(rb_ctx* ctx, const GemmArgs& a) {
     return RB_OK;
   }
   // rows per thread: a slice of K costs a thread TM rows' products and about two rows' worth of reading the features
-  // (a gated tile holds two sets of sums, so it stays smaller)
+  // (a gated tile holds two sets of sums, so it stays smaller).  Where K is too short to be cut, tiles may not fill the GPU, and
+  // what counts is how long one of them takes and how many follow it on an SM (us: 128 x 2048 x 100 with a residual 31 -> 12.5, 1000 x 64 x 64
+  // 25 -> 8.3, 512 x 2048 x 100 33 -> 22, gated 200 x 2048 x 100 30 -> 21).
   constexpr int most = GATED ? 5 : 8;
   const int64_t r16 = (a.m + 15) / 16;
-  auto cost = [&](int t) { return (r16 + t - 1) / t * (t + 2); };
+  const int64_t nt = (a.n + kBN - 1) / kBN, slots = 2 * (int64_t)ctx->sm_count;
+  const bool short_k = (a.k + kBK - 1) / kBK < 8;
+  auto cost = [&](int t) {
+    const int64_t tiles = (r16 + t - 1) / t;
+    return (short_k ? (tiles * nt + slots - 1) / slots : tiles) * (t + 2);
+  };
   int best = 1;
   for (int t = 2; t <= most; ++t)
     if (cost(t) <= cost(best)) best = t;

@@ -168,3 +168,9 @@ def test_float32_products(cuda, m, n, k):
     cuda.synchronize()
     ref = torch.nn.functional.silu(x.double() @ w.double().t()) * (x.double() @ w2.double().t())
     assert float((out.double() - ref).abs().max()) <= 2 * bound(torch.float32, ref, k)
+
+
+# K too short to be cut: as many tiles as fit the GPU at once, then taller ones
+@pytest.mark.parametrize("m,n,k", [(128, 64, 64), (300, 2048, 100), (513, 200, 220), (1000, 64, 8), (700, 6000, 36), (257, 64, 224)])
+def test_float32_products_of_short_rows(cuda, m, n, k):
+    test_float32_products(cuda, m, n, k)

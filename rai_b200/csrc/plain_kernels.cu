@@ -69,9 +69,12 @@ __global__ void gemm_plain_kernel(const T* __restrict__ x, const T* __restrict__
 
 // One block per (token, query head): its 8 warps take every 8th key of the paged cache, each with an online
 // softmax of its own (lanes split head_dim), and their (max, sum, O) states are merged through shared memory.
-// float32 throughout.  Correct for any head_dim <= 32 * NJ.
+// float32 throughout.  Correct for any head_dim <= 32 * NJ.  U keys at a time, so that their rows are on the way together and their
+// sums overlap; their rows are registers, so NJ is no more than the heads need, and many blocks of wide heads take one key at a time.
+// float32, us, with U = 4 and NJ = 8 for all heads up to 256 -> this (one key at a time, NJ = 8): prompts of 200 tokens of 14 heads of 64
+// 74 -> 53 (59), 3 x 77 of 32 heads of 80 105 -> 79 (82), 3 x 200 of 8 heads of 256 131 -> 113 (127); one token and 1000 keys of 64 47 -> 43 (72).
 constexpr int kPlainAttnWarps = 8;
-template <typename T, int NJ>
+template <typename T, int NJ, int U>
 __global__ void __launch_bounds__(kPlainAttnWarps * 32)
 attention_plain_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
                        const int32_t* __restrict__ block_table, const int32_t* __restrict__ seq_lens, int pages_per_seq,
@@ -95,8 +98,6 @@ attention_plain_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, c
   const int first = ext ? first_visible(limit, x.window > 0 ? x.window : 1 << 30, x.chunk) : 0;
   const float slope = ext && x.alibi ? alibi_slope(h, q_heads) : 0.f;
   if (ext) scale *= query_temperature(limit, x.temp_every, x.temp_coef);
-  // U keys at a time, so that their rows are on the way together and their sums overlap
-  constexpr int U = NJ <= 8 ? 4 : 1;
   for (int t0 = first + warp; t0 <= limit; t0 += U * kPlainAttnWarps) {
     T kr[U][NJ], vr[U][NJ];
     bool seen[U], any = false;
@@ -269,12 +270,12 @@ int gemm_simple(rb_ctx* ctx, const GemmArgs& a, int dtype) {
   return fail(RB_ERR_DTYPE, "gemm: dtype %d unsupported", dtype);
 }
 
-template <typename T, int NJ>
+template <typename T, int NJ, int U>
 static int attention_plain_launch(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int batch, int s_new, int q_heads, float scale,
                                   void* out, const AttnExtra* ext, const Packed* pk) {
   const size_t loff = (size_t)layer * c->layer_stride_elems();
   dim3 grid((unsigned)(pk ? pk->rows : batch * s_new), (unsigned)q_heads);
-  attention_plain_kernel<T, NJ><<<grid, kPlainAttnWarps * 32, 0, ctx->stream>>>(
+  attention_plain_kernel<T, NJ, U><<<grid, kPlainAttnWarps * 32, 0, ctx->stream>>>(
       (const T*)q, (const T*)c->k + loff, (const T*)c->v + loff, c->block_table, c->seq_lens, c->pages_per_seq, s_new, q_heads, c->kv_heads,
       c->head_dim, scale, c->window, (T*)out, ext ? 1 : 0, ext ? *ext : AttnExtra(), pk ? *pk : Packed());
   ctx->launches++;
@@ -285,9 +286,14 @@ int attention_simple(rb_ctx* ctx, const void* q, rb_kv_cache* c, int layer, int 
                      float scale, void* out, int dtype, const AttnExtra* ext, const Packed* pk) {
   RB_REQUIRE(dtype == RB_F32 || dtype == RB_BF16, "attention: dtype %d unsupported", dtype);
   RB_REQUIRE(c->head_dim <= 1024, "attention: head_dim %d exceeds 1024", c->head_dim);
-  const bool wide = c->head_dim > 256;
-  const auto run = dtype == RB_F32 ? (wide ? attention_plain_launch<float, 32> : attention_plain_launch<float, 8>)
-                                   : (wide ? attention_plain_launch<__nv_bfloat16, 32> : attention_plain_launch<__nv_bfloat16, 8>);
+  const bool many = (int64_t)(pk ? pk->rows : batch * s_new) * q_heads > 4 * (int64_t)ctx->sm_count;   // four blocks of one key at a time fit an SM
+  const auto go = [&](auto zero) {
+    using T = decltype(zero);
+    const int d = c->head_dim;
+    return d <= 64 ? attention_plain_launch<T, 2, 4> : d <= 96 ? attention_plain_launch<T, 3, 4> : d <= 128 ? attention_plain_launch<T, 4, 4>
+         : d > 256 ? attention_plain_launch<T, 32, 1> : many ? attention_plain_launch<T, 8, 1> : attention_plain_launch<T, 8, 4>;
+  };
+  const auto run = dtype == RB_F32 ? go(0.f) : go(__nv_bfloat16());
   return run(ctx, q, c, layer, batch, s_new, q_heads, scale, out, ext, pk);
 }
 

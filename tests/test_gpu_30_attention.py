@@ -151,3 +151,9 @@ def test_append_beyond_capacity_is_rejected(cuda):
     with pytest.raises(_lib.RaiB200Error):
         cache.set_len(2, 1)
     cache.close()
+
+
+@pytest.mark.parametrize("d", [24, 64, 72, 96, 104, 128, 136, 256])
+def test_float32_heads_of_every_register_count(cuda, d):
+    """The float32 kernel has as many columns of a lane as heads need: on both sides of 64, 96 and 128, and the largest."""
+    test_rope_append_attention_matches_oracle(cuda, torch.float32, 4, 2, d, d, 2, 45, 2)

@@ -141,6 +141,7 @@ extern "C" int32_t rb_sync(rb_ctx* ctx) {
       RB_CUDA(cudaMemset(ctx->argmax_count, 0, kArgmaxRows * sizeof(unsigned int)));
       RB_CUDA(cudaMemset(ctx->gemm_tile_count, 0, 2 * kGemmMaxReduceTiles * sizeof(uint32_t)));
       for (uint32_t* f : ctx->pair_flags) RB_CUDA(cudaMemset(f, 0, kPairFlagBytes));
+      for (uint32_t* f : ctx->step_flags) RB_CUDA(cudaMemset(f, 0, kStepFlagBytes));
       RB_CUDA(cudaStreamSynchronize(nullptr));  // the words are clear before any stream's next launch
     }
     return fail(code, "device-side check failed: code %d at 0x%x (detail %u, %u)", code, w[1], w[2], w[3]);

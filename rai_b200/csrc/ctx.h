@@ -16,6 +16,7 @@
 constexpr int kPairClusters = 74;
 constexpr size_t kPairSlabBytes = (size_t)kPairClusters * 4 * 128 * 256 * sizeof(float);
 constexpr size_t kPairFlagBytes = (size_t)kPairClusters * 4 * 8 * sizeof(uint32_t);
+constexpr size_t kStepFlagBytes = 256;   // step.cu: arrivals at the barriers of a launch; CTAs that have left it
 struct PairSpace {
   float* slabs = nullptr;
   uint32_t* flags = nullptr;
@@ -40,6 +41,7 @@ struct rb_ctx {
   uint32_t* gemm_tile_count = nullptr;  // [2][kGemmMaxReduceTiles] arrival / done counters of those GEMMs, self-resetting
   const PairSpace* pair_space = nullptr;    // lent for the call at hand; NULL: products are not cut
   std::vector<uint32_t*> pair_flags;        // of every PairSpace there is, for rb_sync to clear
+  std::vector<uint32_t*> step_flags;        // barriers of step.cu, likewise
   long long wait_budget_cycles = 2000000000LL;  // give-up time of a device-side wait for ANOTHER GPU (rb_set_wait_budget_us)
   // Waits inside one kernel (operand rings, accumulators, sibling blocks) may begin before the kernel's predecessor
   // has finished, and that predecessor may itself be waiting for a peer: they get four times the budget, so that
@@ -157,6 +159,8 @@ struct ProfScope {
 
 // Internal launchers shared between api.cu and model.cu (defined next to their kernels).
 int tmap_2d_bf16(rb_ctx* ctx, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows, CUtensorMap* out);
+// the same matrix as slices of 64 columns (cols % 64 == 0): coordinates (0, row, slice), boxes of box_rows x box_slices
+int tmap_slices_bf16(const void* base, int64_t rows, int64_t cols, int box_rows, int box_slices, CUtensorMap* out);
 
 struct GemmArgs {
   const void* x = nullptr;      // [M, K]

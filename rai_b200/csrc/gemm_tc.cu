@@ -733,6 +733,21 @@ int tmap_2d_bf16(rb_ctx* ctx, const void* base, int64_t rows, int64_t cols, int6
   return RB_OK;
 }
 
+int tmap_slices_bf16(const void* base, int64_t rows, int64_t cols, int box_rows, int box_slices, CUtensorMap* out) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(RB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || cols % 64)
+    return fail(RB_ERR_INVALID, "GEMM operand must be 16-byte aligned with rows of whole 64-column slices");
+  const cuuint64_t dims[3] = {64, (cuuint64_t)rows, (cuuint64_t)(cols / 64)};
+  const cuuint64_t strides[2] = {(cuuint64_t)cols * 2, 128};
+  const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, (cuuint32_t)box_slices}, estr[3] = {1, 1, 1};
+  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(RB_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
+  return RB_OK;
+}
+
 // How many ways to split K for a decode-sized launch that would otherwise leave most SMs idle (1 = do not split).
 int gemm_reserve_scratch(rb_ctx* ctx, size_t bytes);
 

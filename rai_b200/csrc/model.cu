@@ -304,6 +304,7 @@ int last_rows_logits(rb_model* m, int seq, const int32_t* rows_dev, int n) {
 int forward_body(rb_model* m, const uint32_t* tokens, int batch, int seq, void* logits_out, const int32_t* rows_dev = nullptr,
                  int n_rows = -1, const int32_t* new_lens = nullptr, const Packed* pk = nullptr);
 int finish_logits(rb_model* m, int batch, int seq, void* logits_out, const int32_t* rows_dev, int n_rows);
+int copy_logits(rb_model* m, int first, int n, void* logits_out);
 
 // act = activation(x . W1^T [+ b1]) [* (x . Wup^T)]  -- the first half of MLP::fwd.  When the fused kernel
 // would leave most SMs idle (decode-sized rows and few 128-row weight tiles, i.e. small or sharded
@@ -432,6 +433,12 @@ int forward_body(rb_model* m, const uint32_t* tokens, int batch, int seq, void* 
   const float emb_scale = c.arch == RB_ARCH_GEMMA ? sqrtf((float)H) : 1.0f;  // gemma.rs:379
   RB_TRY(rb_embed_gather(ctx, m->embed, c.dtype, c.vocab_size, H, tokens, rows, emb_scale, m->h));
 
+  if (seq == 1 && !pk && step_takes(m, batch)) {
+    RB_TRY(step_forward(m, batch, !rows_dev));
+    if (rows_dev) return finish_logits(m, batch, seq, logits_out, rows_dev, n_rows);
+    return copy_logits(m, 0, batch, logits_out);
+  }
+
   const float scale = 1.0f / sqrtf((float)d);
   const int L = c.num_hidden_layers;
   Pending pend;
@@ -484,16 +491,21 @@ int forward_body(rb_model* m, const uint32_t* tokens, int batch, int seq, void* 
   return finish_logits(m, batch, seq, logits_out, rows_dev, n_rows);
 }
 
+int copy_logits(rb_model* m, int first, int n, void* logits_out) {
+  const size_t row_bytes = (size_t)m->cfg.vocab_size * dtype_size(m->logits_dtype);
+  if (logits_out && logits_out != m->logits)
+    RB_CUDA(cudaMemcpyAsync((char*)logits_out + (size_t)first * row_bytes, m->logits, (size_t)n * row_bytes, cudaMemcpyDeviceToDevice,
+                            m->ctx->stream));
+  return RB_OK;
+}
+
 // Final norm and vocabulary product of the wanted rows, at most max_batch at a time.
 int finish_logits(rb_model* m, int batch, int seq, void* logits_out, const int32_t* rows_dev, int n_rows) {
   const rb_model_config& c = m->cfg;
-  const size_t row_bytes = (size_t)c.vocab_size * dtype_size(m->logits_dtype);
   for (int r0 = 0; r0 < n_rows; r0 += c.max_batch) {
     const int n = std::min(n_rows - r0, (int)c.max_batch);
     RB_TRY(last_rows_logits(m, seq, rows_dev ? rows_dev + r0 : nullptr, n));
-    if (logits_out && logits_out != m->logits)
-      RB_CUDA(cudaMemcpyAsync((char*)logits_out + (size_t)r0 * row_bytes, m->logits, (size_t)n * row_bytes, cudaMemcpyDeviceToDevice,
-                              m->ctx->stream));
+    RB_TRY(copy_logits(m, r0, n, logits_out));
   }
   return RB_OK;
 }
@@ -795,6 +807,7 @@ extern "C" int32_t rb_model_create(rb_ctx* ctx, const rb_model_config* cfg, rb_m
     m->scratch_floats = (size_t)16 * rows * std::max(m->nqkv_l, H);
     W(m->scratch_floats * sizeof(float), (void**)&m->scratch);
   }
+  if (st == RB_OK) st = step_reserve(m);
   if (st != RB_OK) { rb_model_destroy(m); return st; }
 #ifdef RB_DEBUG_AIDS
   {
@@ -834,6 +847,9 @@ extern "C" int32_t rb_model_destroy(rb_model* m) {
   if (m->cache) rb_kv_cache_destroy(m->cache);
   std::vector<uint32_t*>& flags = m->ctx->pair_flags;
   flags.erase(std::remove(flags.begin(), flags.end(), m->pair_space.flags), flags.end());
+  std::vector<uint32_t*>& steps = m->ctx->step_flags;
+  steps.erase(std::remove(steps.begin(), steps.end(), m->step_flags), steps.end());
+  step_plan_free(m->step_plan);
   for (void* p : m->owned) rb_free(m->ctx, p);
   delete m;
   return RB_OK;
@@ -1264,11 +1280,12 @@ int sample_tokens(rb_model* m, int batch, uint32_t* out) {
 }
 
 // Whatever host-side state shapes the launches of a decode step: a captured step is reused only
-// while this stays the same (today: how many KV splits the attention uses).
+// while this stays the same (which kernels the step takes, and how many KV splits the attention uses).
 int decode_plan(rb_model* m, int batch) {
   if (m->layered) return layered_decode_plan(m, batch);
   int max_len = 0;
   for (int b = 0; b < batch; ++b) max_len = std::max(max_len, m->cache->host_lens[b]);
+  if (step_takes(m, batch)) return 0;   // (it reads all lengths on the device)
   return attention_decode_splits(m->ctx, batch, m->nkv_l, m->nq_l / m->nkv_l, max_len, m->d);
 }
 

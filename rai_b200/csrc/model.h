@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "ctx.h"
+#include "step.h"
 
 namespace rb {
 
@@ -102,6 +103,8 @@ struct rb_model {
   int32_t* last_rows = nullptr;           // the rows of a call whose logits are wanted [max_tokens]
   std::vector<int32_t> last_rows_host;    // outlives the asynchronous upload
   PairSpace pair_space;      // of prompt products cut along K
+  rb::StepPlan* step_plan = nullptr;   // of steps that run as one kernel (step.cu); NULL: none do
+  uint32_t* step_flags = nullptr;
   float* scratch = nullptr;  // split-K partials
   size_t scratch_floats = 0;
   void* comm = nullptr;

@@ -1,0 +1,100 @@
+"""Single-token steps of up to eight sequences that run as one kernel (layers of more than 96 MB): every family and head size it takes, sizes
+that no share of 148 divides, contexts around the edges of key tiles, pairs cut into pieces, sequences of different lengths - against
+the oracle, with the tolerance of the other model tests; the replayed step against plain ones; and who takes the kernel."""
+import numpy as np
+import pytest
+import torch
+
+import util
+from rai_b200 import _lib, configs, synth
+from rai_b200.models import Model
+
+pytestmark = pytest.mark.gpu
+
+FAMILIES = {
+    # heads of 64, one for keys and values, group 31 > 16 is not taken: 30 heads in two groups of 15; rows of 1920 = 148 * 13 - 4
+    "qwen2-64": ("tiny-qwen2", dict(hidden_size=1920, num_attention_heads=30, num_key_value_heads=2, intermediate_size=8896)),
+    "qwen2-128": ("tiny-qwen2", dict(hidden_size=1792, num_attention_heads=14, num_key_value_heads=2, intermediate_size=9536)),
+    "qwen2-128-tied": ("tiny-qwen2-tied", dict(hidden_size=2560, num_attention_heads=20, num_key_value_heads=20, intermediate_size=6464)),
+    "phi2-80": ("tiny-phi2", dict(hidden_size=2560, num_attention_heads=32, num_key_value_heads=32, intermediate_size=10304)),
+    "phi3-96": ("tiny-phi3", dict(hidden_size=2304, num_attention_heads=24, num_key_value_heads=24, intermediate_size=7488)),
+    "gemma-128": ("tiny-gemma", dict(hidden_size=2048, num_attention_heads=16, num_key_value_heads=1, head_dim=128, intermediate_size=8256)),
+}
+
+
+def _config(family, layers=2):
+    name, sizes = FAMILIES[family]
+    cfg = configs.get(name)
+    cfg.update(sizes, num_hidden_layers=layers, vocab_size=1031, max_position_embeddings=1024)
+    return cfg
+
+
+@pytest.mark.parametrize("family", list(FAMILIES))
+@pytest.mark.parametrize("lens", [[1], [63], [700], [64, 65], [2, 63, 200], [128] * 4, [5, 129, 64, 300, 1, 191, 66], [40] * 8])
+def test_steps_match_the_oracle(cuda, family, lens):
+    cfg = _config(family)
+    w = synth.weights(cfg, 21)
+    oracle = util.build_oracle(cfg, w)
+    b, steps = len(lens), 3
+    m = Model(cfg, _lib.BF16, cuda, b, 768, sum(lens) + 8 * b * max(lens))
+    m.update_params(w)
+    fed = synth.prompt(cfg, b, max(lens) + steps, 22).astype(np.int32)
+    prompts = np.zeros((b, max(lens)), np.int32)
+    for i, n in enumerate(lens):
+        prompts[i, :n] = fed[i, :n]
+    m.forward_ragged(prompts, lens)
+    got = []
+    for t in range(steps):
+        ids = np.stack([fed[i, n + t:n + t + 1] for i, n in enumerate(lens)])
+        before = cuda.launch_count()
+        if len(set(lens)) == 1:
+            got.append(m.forward(ids, lens[0] + t).reshape(b, -1).float().cpu())
+        else:
+            got.append(m.forward_rows(ids, None, range(b)).reshape(b, -1).float().cpu())
+        assert cuda.launch_count() - before <= 6   # (a layer of kernels of its own would be seven)
+    for i, n in enumerate(lens):
+        oracle.clear_kv_cache()
+        oracle.forward(torch.from_numpy(fed[i:i + 1, :n].astype(np.int64)), 0)
+        for t in range(steps):
+            want = oracle.forward(torch.from_numpy(fed[i:i + 1, n + t:n + t + 1].astype(np.int64)), n + t).reshape(-1)
+            assert util.logit_error(got[t][i], want) <= 2e-2, (i, t)
+    m.close()
+
+
+@pytest.mark.parametrize("family", ["qwen2-128", "phi2-80"])
+def test_replayed_steps_are_the_plain_ones_and_the_next_context_crosses_a_tile(cuda, family):
+    """Eight replays of the captured step (from 60 keys over the edge of the tile) give the tokens and, in one more step, the bits of plain calls."""
+    cfg = _config(family)
+    b, n, steps = 3, 60, 8
+    m = Model(cfg, _lib.BF16, cuda, b, 128, b * n)
+    m.update_params(synth.weights(cfg, 23))
+    ids = synth.prompt(cfg, b, n, 24).astype(np.int32)
+
+    def best(logits):   # of equal logits (8 bits tell few of a thousand apart) the last, which is what the device's sampling takes
+        logits = logits.reshape(b, -1).float().cpu()
+        return np.array([[int((row == row.max()).nonzero()[-1])] for row in logits], np.int32)
+
+    plain = [best(m.forward(ids, 0))]
+    for t in range(steps):
+        plain.append(best(m.forward(plain[-1], n + t)))
+    last = m.forward(plain[-1], n + steps).float().cpu()
+    m.clear_kv_cache()
+    loop = m.decode_loop(torch.from_numpy(best(m.forward(ids, 0)).reshape(-1)).cuda(), n, steps).cpu().numpy()
+    assert (loop == np.stack([p.reshape(-1) for p in plain[1:]])).all()
+    again = m.forward(loop[-1].reshape(b, 1), n + steps).float().cpu()
+    assert torch.equal(last, again)
+    m.close()
+
+
+@pytest.mark.parametrize("batch,context,one", [(8, 64, True), (9, 64, False), (8, 1450, True), (8, 1550, False)])
+def test_who_takes_the_kernel(cuda, batch, context, one):
+    """Up to eight sequences, and up to three quarters of a layer's weights (146 MB) in cached bytes (9.2 KB a token)."""
+    cfg = _config("phi3-96")
+    cfg["max_position_embeddings"] = 2048
+    m = Model(cfg, _lib.BF16, cuda, batch, 1600, batch)
+    m.update_params(synth.weights(cfg, 25))
+    _lib.call("rb_kv_cache_set_len", _lib.lib().rb_model_kv_cache(m._m), batch, context)
+    before = cuda.launch_count()
+    m.forward(np.ones((batch, 1), np.int32), context)
+    assert (cuda.launch_count() - before <= 6) == one
+    m.close()

@@ -6,9 +6,9 @@
 // layer.  Here one CTA stays on every SM and the phases of a layer follow one another through grid-wide barriers (five a layer, 2 us from the
 // last arrival to the first product), while the copies of weights and cached keys and values, which depend on nothing, run ahead through
 // all of them: a ring of shared memory (190 KB an SM, 4.5 us of HBM over the GPU) takes the tiles of the next phase while this one
-// waits.  us per step of 8 layers, seven launches a layer -> here: phi2 (157 MB a layer) 1 x 64 keys 515 -> 384, 8 x 512 577 -> 521;
-// phi3-mini (226 MB) 1 x 2048 619 -> 516, 4 x 2048 704 -> 627; qwen2-7b (466 MB) 1 x 128 959 -> 910.  A layer of phi3-mini with 4 x 2048
-// keys takes 70 us, of which 50 are its 326 MB at the copy rate; inside the phases HBM delivers 6 TB/s (5 in attention).
+// waits.  us per step of 8 layers, seven launches a layer -> here: phi2 (157 MB a layer) 1 x 64 keys 515 -> 383, 8 x 512 576 -> 508;
+// phi3-mini (226 MB) 1 x 2048 613 -> 507, 4 x 2048 701 -> 613; qwen2-7b (466 MB) 1 x 128 957 -> 913.  A layer of phi3-mini with 4 x 2048
+// keys takes 69 us, of which 50 are its 326 MB at the copy rate; inside the phases HBM delivers 6 TB/s (5 in attention).
 //
 //   warp 8      weights, keys and values: TMA tiles into the ring in the order of the program, whatever phase the rest is in
 //   warps 9, 10 wait at the barriers; then the activations that belong to each weight tile (a few KB from L2) into the same slot
@@ -327,8 +327,8 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
               uint64_t* bar = &sh.full[r.slot];
               ptx::mbar_expect_tx(bar, C::kTileBytes);
 #pragma unroll
-              for (int cb = 0; cb < C::kBlocks; ++cb)
-                ptx::tma_load_2d(ring + r.slot * slot_bytes + cb * (C::kKeys * 128), j & 1 ? &p.v : &p.k, bar, cb * 64, y);
+              for (int cb = 0; cb < C::kBlocks; ++cb)   // (read once a step: L2 is for what the CTAs share, 8 x 512 keys of phi2 521 -> 508 us)
+                ptx::tma_load_2d_hint(ring + r.slot * slot_bytes + cb * (C::kKeys * 128), j & 1 ? &p.v : &p.k, bar, cb * 64, y, policy);
               ptx::mbar_arrive(bar);   // (in the place of the activations)
               r.pass(slots);
             }

@@ -1119,7 +1119,7 @@ int step_reserve(rb_model* m) {
 }
 
 // Up to eight sequences, and no more cached bytes than three quarters of the weights': the attention phase reads K and V at 5 TB/s, a launch
-// of its own at 5.5.  us per step of 8 layers, as launches -> here, and cached bytes to weights: phi3-mini 1 x 2048 keys 619 -> 516 (0.11),
+// of its own at 5.5.  us per step of 8 layers, as launches -> here (K and V without the L2 hint on both sides), and cached bytes to weights: phi3-mini 1 x 2048 keys 619 -> 516 (0.11),
 // 4 x 2048 704 -> 627 (0.44), 8 x 200 603 -> 537 (0.09), 8 x 2048 813 -> 828 (0.89); phi2 1 x 64 515 -> 384, 8 x 512 577 -> 521 (0.27),
 // 8 x 1500 672 -> 670 (0.78); qwen2-7b 1 x 128 959 -> 910, 8 x 2048 1063 -> 1039 (0.07).  With sixteen sequences (two eights per product)
 // every one of these was slower: phi3-mini 16 x 200 675 -> 706, qwen2-7b 16 x 2048 1086 -> 1164.

@@ -787,6 +787,10 @@ int32_t rb_model_finished(rb_model* m, int32_t batch, uint8_t* flags_host);
  * a captured CUDA graph, 0 when they are issued launch by launch.  No counterpart in the reference. */
 int32_t rb_model_decode_graph_active(rb_model* m);
 int32_t rb_model_clear_kv_cache(rb_model* m);
+/* Test hook: the next single-token step of this model, if it runs as one kernel, waits for blocks that never arrive, gives up after the
+ * wait budget and reports RB_ERR_TIMEOUT; rb_sync makes the model fit for use again.  RB_ERR_INVALID for a model none of whose
+ * steps run so.  No counterpart in the reference. */
+int32_t rb_selftest_spoil_step(rb_model* m);
 rb_kv_cache* rb_model_kv_cache(rb_model* m);
 /* Number of kernels the library launched on this context since creation (self-reported count). */
 int64_t rb_launch_count(rb_ctx* ctx);

@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "ctx.h"
+#include "model.h"
 #include "ptx.cuh"
 
 namespace rb {
@@ -195,4 +196,9 @@ extern "C" int32_t rb_selftest_pair_linear(rb_ctx* ctx, const void* x, const voi
   RB_CUDA(cudaMemcpy(words.data(), flags.p, kPairFlagBytes, cudaMemcpyDeviceToHost));
   if (std::any_of(words.begin(), words.end(), [](uint32_t v) { return v != 0u; })) return fail(RB_ERR_CUDA, "rb_selftest_pair_linear: a flag was left raised");
   return RB_OK;
+}
+
+extern "C" int32_t rb_selftest_spoil_step(rb_model* m) {
+  RB_REQUIRE(m, "rb_selftest_spoil_step: null model");
+  return step_spoil(m);
 }

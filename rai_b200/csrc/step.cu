@@ -277,7 +277,11 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
   if (warp == kWorkWarps) {
     if (lane == 0) {
       const uint64_t policy = ptx::policy_evict_first();
-      auto acquire = [&]() { return ok = ptx::mbar_wait(&sh.empty[r.slot], r.parity ^ 1u, abort_flag, p.wait_cycles); };
+      // (A slot that was given back without having been waited for must not be armed again: its barrier may still expect what was asked for.
+      // Whoever gives it back so has seen the flag, and who acquires it sees it, too.)
+      auto acquire = [&]() {
+        return ok = ptx::mbar_wait(&sh.empty[r.slot], r.parity ^ 1u, abort_flag, p.wait_cycles) && *abort_flag == 0;
+      };
 #pragma unroll 1
       for (int l = 0; l <= p.layers && ok; ++l) {
 #pragma unroll 1
@@ -336,11 +340,6 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
           }
         }
       }
-      if (!ok) {
-        // somebody gave up; copies under way end within microseconds, and the CTA must not leave before them
-        const long long t0 = clock64();
-        while (clock64() - t0 < 2000000) {}
-      }
     }
   }
   // ================================================================ barriers and activations
@@ -386,7 +385,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
 #pragma unroll 1
               for (int k = 0; k < stages; ++k) {
                 if ((r.slot & 1) == turn && ok) {
-                  ok = ptx::mbar_wait(&sh.empty[r.slot], r.parity ^ 1u, abort_flag, p.wait_cycles);
+                  ok = ptx::mbar_wait(&sh.empty[r.slot], r.parity ^ 1u, abort_flag, p.wait_cycles) && *abort_flag == 0;   // (as above)
                   uint64_t* bar = &sh.full[r.slot];
                   if (ok) {
                     ptx::mbar_expect_tx(bar, bytes);
@@ -416,7 +415,9 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
     auto arrive = [&]() {   // this CTA's part of the phase is in memory, for copies to read, too
       asm volatile("fence.proxy.async.global;" ::: "memory");
       work_sync();
-      if (tid == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.flags) : "memory");
+      // (A CTA that has given up waits for nothing more, and must not be counted: other CTAs' barriers would open before their own attention is
+      // through, and activations asked for then would arrive on barriers of slots in an older use.)
+      if (tid == 0 && *abort_flag == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.flags) : "memory");
     };
     auto wait_go = [&]() { ptx::mbar_wait(&sh.go, gone & 1u, abort_flag, p.wait_cycles); ++gone; };
     // (A parity tells a slot's use from the one before it, not from the one before that: who does not read every slot in turn first sees that
@@ -991,11 +992,17 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
         if (op != kHead && (serial || op != kQkv)) arrive();
       }
     }
-    if (tid == 0 && *abort_flag) { p.status[0] = (uint32_t)(-RB_ERR_TIMEOUT); p.status[1] = 0x57E9u; p.status[2] = (uint32_t)cta; }
+  }
+  __syncwarp();
+  __syncthreads();   // no role asks for a copy any more
+  if (threadIdx.x == 0 && sh.abort) {
+    // Whoever gave up, the others went on without waiting: copies that any of the three asking warps had issued may be under way.  They
+    // end within microseconds, and the CTA must not leave before them.
+    p.status[0] = (uint32_t)(-RB_ERR_TIMEOUT); p.status[1] = 0x57E9u; p.status[2] = (uint32_t)cta;
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000) {}
   }
   // the last CTA to leave, when nobody waits any more, puts the barriers' count back
-  __syncwarp();
-  __syncthreads();
   if (threadIdx.x == 0 && atomicInc(p.flags + 32, (uint32_t)ctas - 1u) == (uint32_t)ctas - 1u) *p.flags = 0u;
 }
 
@@ -1128,6 +1135,16 @@ bool step_takes(const rb_model* m, int batch) {
   double tokens = 0;
   for (int b = 0; b < batch; ++b) tokens += m->cache->host_lens[b];
   return tokens * m->step_plan->token_bytes <= 0.75 * m->step_plan->layer_bytes;
+}
+
+int step_spoil(rb_model* m) {
+  RB_REQUIRE(m->step_plan, "this model has no resident steps");
+  // (behind by more than all arrivals of a step, 160 x 5 x 40 and some.  Never ahead: a barrier that opens early lets activations into
+  // slots of an older use, and an arrival that a mbarrier does not expect is a launch failure.)
+  const uint32_t far = 0u - (1u << 20);
+  RB_CUDA(cudaStreamSynchronize(m->ctx->stream));
+  RB_CUDA(cudaMemcpy(m->step_flags, &far, sizeof(far), cudaMemcpyHostToDevice));
+  return RB_OK;
 }
 
 int step_forward(rb_model* m, int batch, bool want_head) {

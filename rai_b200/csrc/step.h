@@ -12,5 +12,7 @@ void step_plan_free(StepPlan* plan);
 bool step_takes(const rb_model* m, int batch);
 // From the embedded rows in m->h to m->logits (want_head), or to the final rows of the stream in m->h alone.
 int step_forward(rb_model* m, int batch, bool want_head);
+// Test hook: the model's next step waits for arrivals that never come, and gives up.
+int step_spoil(rb_model* m);
 
 }  // namespace rb

@@ -1,6 +1,8 @@
 """Single-token steps of up to eight sequences that run as one kernel (layers of more than 96 MB): every family and head size it takes, sizes
 that no share of 148 divides, contexts around the edges of key tiles, pairs cut into pieces, sequences of different lengths - against
 the oracle, with the tolerance of the other model tests; the replayed step against plain ones; and who takes the kernel."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -97,4 +99,32 @@ def test_who_takes_the_kernel(cuda, batch, context, one):
     before = cuda.launch_count()
     m.forward(np.ones((batch, 1), np.int32), context)
     assert (cuda.launch_count() - before <= 6) == one
+    m.close()
+
+
+@pytest.mark.parametrize("family", ["qwen2-128", "phi2-80"])
+def test_a_step_that_gives_up_says_so_and_the_next_ones_are_right(cuda, family):
+    """Barriers that never open: every role stops waiting after the budget, the block stays until its copies have landed, the host learns of
+    it, and the same step afterwards gives the same bits as ever."""
+    cfg = _config(family)
+    b, n = 3, 200
+    m = Model(cfg, _lib.BF16, cuda, b, 256, b * n)
+    m.update_params(synth.weights(cfg, 27))
+    ids, token = synth.prompt(cfg, b, n, 28).astype(np.int32), np.array([[1], [2], [3]], np.int32)
+
+    def prompt_and_step():
+        m.clear_kv_cache()
+        m.forward(ids, 0)
+        return lambda: m.forward(token, n).float().cpu()
+
+    want = prompt_and_step()()
+    step = prompt_and_step()
+    _lib.call("rb_set_wait_budget_us", cuda.ctx, 500)
+    try:
+        _lib.call("rb_selftest_spoil_step", m._m)
+        with pytest.raises(_lib.RaiB200Error, match="0x57e9"):
+            step()
+    finally:
+        _lib.call("rb_set_wait_budget_us", cuda.ctx, 1000000)
+    assert torch.equal(prompt_and_step()(), want)
     m.close()

@@ -791,6 +791,9 @@ int32_t rb_model_clear_kv_cache(rb_model* m);
  * wait budget and reports RB_ERR_TIMEOUT; rb_sync makes the model fit for use again.  RB_ERR_INVALID for a model none of whose
  * steps run so.  No counterpart in the reference. */
 int32_t rb_selftest_spoil_step(rb_model* m);
+/* Test hook: the next launch of such a step fails as it does where the grid does not fit into the SMs that the stream may use; that step
+ * and all later ones of the model run as separate launches.  RB_ERR_INVALID as above.  No counterpart in the reference. */
+int32_t rb_selftest_refuse_step(rb_model* m);
 rb_kv_cache* rb_model_kv_cache(rb_model* m);
 /* Number of kernels the library launched on this context since creation (self-reported count). */
 int64_t rb_launch_count(rb_ctx* ctx);

@@ -303,6 +303,7 @@ extern "C" {
     pub fn rb_model_decode_graph_active(m: *mut rb_model) -> i32;
     pub fn rb_model_clear_kv_cache(m: *mut rb_model) -> i32;
     pub fn rb_selftest_spoil_step(m: *mut rb_model) -> i32;
+    pub fn rb_selftest_refuse_step(m: *mut rb_model) -> i32;
     pub fn rb_model_kv_cache(m: *mut rb_model) -> *mut rb_kv_cache;
     pub fn rb_launch_count(ctx: *mut rb_ctx) -> i64;
     pub fn rb_profile_start(ctx: *mut rb_ctx) -> i32;

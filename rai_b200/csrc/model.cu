@@ -434,9 +434,10 @@ int forward_body(rb_model* m, const uint32_t* tokens, int batch, int seq, void* 
   RB_TRY(rb_embed_gather(ctx, m->embed, c.dtype, c.vocab_size, H, tokens, rows, emb_scale, m->h));
 
   if (seq == 1 && !pk && step_takes(m, batch)) {
-    RB_TRY(step_forward(m, batch, !rows_dev));
-    if (rows_dev) return finish_logits(m, batch, seq, logits_out, rows_dev, n_rows);
-    return copy_logits(m, 0, batch, logits_out);
+    bool ran = false;
+    RB_TRY(step_forward(m, batch, !rows_dev, &ran));
+    if (ran && rows_dev) return finish_logits(m, batch, seq, logits_out, rows_dev, n_rows);
+    if (ran) return copy_logits(m, 0, batch, logits_out);
   }
 
   const float scale = 1.0f / sqrtf((float)d);

@@ -202,3 +202,8 @@ extern "C" int32_t rb_selftest_spoil_step(rb_model* m) {
   RB_REQUIRE(m, "rb_selftest_spoil_step: null model");
   return step_spoil(m);
 }
+
+extern "C" int32_t rb_selftest_refuse_step(rb_model* m) {
+  RB_REQUIRE(m, "rb_selftest_refuse_step: null model");
+  return step_refuse(m);
+}

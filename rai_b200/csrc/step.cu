@@ -1023,13 +1023,14 @@ StepShare share_rows(int n, int k, bool two, int ctas) {
 }
 
 template <int D>
-int launch(rb_ctx* ctx, const StepParams& p, size_t smem) {
-  static bool attr_set[64] = {};  // the attribute belongs to the (kernel, device) pair
-  bool& set = attr_set[ctx->device & 63];
-  if (!set) {
-    RB_CUDA(cudaFuncSetAttribute(step_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem));
-    set = true;
-  }
+int blocks_per_sm(size_t smem, int* n) {
+  RB_CUDA(cudaFuncSetAttribute(step_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem));
+  RB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, step_kernel<D>, kThreads, smem));
+  return RB_OK;
+}
+
+template <int D>
+cudaError_t launch(rb_ctx* ctx, const StepParams& p, size_t smem) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ctx->sm_count);
   cfg.blockDim = dim3(kThreads);
@@ -1040,9 +1041,7 @@ int launch(rb_ctx* ctx, const StepParams& p, size_t smem) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  RB_CUDA(cudaLaunchKernelEx(&cfg, step_kernel<D>, p));
-  ctx->launches++;
-  return RB_OK;
+  return cudaLaunchKernelEx(&cfg, step_kernel<D>, p);
 }
 
 }  // namespace
@@ -1051,6 +1050,7 @@ int launch(rb_ctx* ctx, const StepParams& p, size_t smem) {
 struct StepPlan {
   StepParams p{};
   size_t smem = 0;
+  bool refused = false;                      // (test hook)
   double layer_bytes = 0, token_bytes = 0;   // weights of a layer; keys and values of a token in it
 };
 void step_plan_free(StepPlan* plan) { delete plan; }
@@ -1090,7 +1090,16 @@ int step_reserve(rb_model* m) {
   const size_t rest = (size_t)p.merge_floats * 4 + (size_t)kRows * p.share[kOut].rows * 4 + 4 * d + (size_t)group * (d + 8) * 2 + 1024;
   p.slots = std::min<int>(kMaxSlots, (int)((kMostSmem - rest) / p.slot_bytes)) & ~1;
   plan->smem = rest + (size_t)p.slots * p.slot_bytes;
-  if (p.slots < kWorkWarps) { delete plan; m->step_plan = nullptr; return RB_OK; }
+  // (a LayerNorm is a row per CTA; the launch is all of the grid or nothing, so a device, or a share of one, without room for it has no plan)
+  int cooperative = 0, per_sm = 0;
+  RB_CUDA(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, ctx->device));
+  switch (d) {
+    case 64: RB_TRY(blocks_per_sm<64>(plan->smem, &per_sm)); break;
+    case 80: RB_TRY(blocks_per_sm<80>(plan->smem, &per_sm)); break;
+    case 96: RB_TRY(blocks_per_sm<96>(plan->smem, &per_sm)); break;
+    default: RB_TRY(blocks_per_sm<128>(plan->smem, &per_sm));
+  }
+  if (p.slots < kWorkWarps || ctas < kRows || !cooperative || per_sm < 1) { delete plan; m->step_plan = nullptr; return RB_OK; }
   for (int l = 0; l < p.layers; ++l) {
     const LayerW& w = m->layers[l];
     p.layer[l] = {(const bf16*)w.qkv_b, (const bf16*)w.o_b, (const bf16*)w.fc1_b, (const bf16*)w.down_b,
@@ -1147,7 +1156,13 @@ int step_spoil(rb_model* m) {
   return RB_OK;
 }
 
-int step_forward(rb_model* m, int batch, bool want_head) {
+int step_refuse(rb_model* m) {
+  RB_REQUIRE(m->step_plan, "this model has no resident steps");
+  m->step_plan->refused = true;
+  return RB_OK;
+}
+
+int step_forward(rb_model* m, int batch, bool want_head, bool* ran) {
   rb_ctx* ctx = m->ctx;
   StepParams& p = m->step_plan->p;
   const size_t smem = m->step_plan->smem;
@@ -1166,12 +1181,26 @@ int step_forward(rb_model* m, int batch, bool want_head) {
     flops += 4.0 * p.layers * m->cache->host_lens[b] * p.q_heads * m->d;
   }
   ProfScope prof(ctx, RB_PROF_GEMM, bytes, flops);
-  switch (m->d) {
-    case 64: return launch<64>(ctx, p, smem);
-    case 80: return launch<80>(ctx, p, smem);
-    case 96: return launch<96>(ctx, p, smem);
-    default: return launch<128>(ctx, p, smem);
+  cudaError_t e = cudaErrorCooperativeLaunchTooLarge;
+  if (!m->step_plan->refused) {
+    switch (m->d) {
+      case 64: e = launch<64>(ctx, p, smem); break;
+      case 80: e = launch<80>(ctx, p, smem); break;
+      case 96: e = launch<96>(ctx, p, smem); break;
+      default: e = launch<128>(ctx, p, smem);
+    }
   }
+  *ran = e == cudaSuccess;
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported) {
+    // fewer SMs than the device has (a stream of a part of them): nothing has run, and this model's steps are launches from now on
+    cudaGetLastError();
+    step_plan_free(m->step_plan);
+    m->step_plan = nullptr;
+    return RB_OK;
+  }
+  RB_CUDA(e);
+  ctx->launches++;
+  return RB_OK;
 }
 
 }  // namespace rb

@@ -128,3 +128,35 @@ def test_a_step_that_gives_up_says_so_and_the_next_ones_are_right(cuda, family):
         _lib.call("rb_set_wait_budget_us", cuda.ctx, 1000000)
     assert torch.equal(prompt_and_step()(), want)
     m.close()
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_a_refused_launch_falls_back_to_the_kernels_of_other_steps(cuda, captured):
+    """All blocks or none: where the launch is refused, the step runs as launches of its own, and so do all later ones."""
+    cfg = _config("phi3-96")
+    b, n, steps = 2, 70, 5
+    w = synth.weights(cfg, 31)
+    m = Model(cfg, _lib.BF16, cuda, b, 128, b * n)
+    m.update_params(w)
+    ids = synth.prompt(cfg, b, n, 32).astype(np.int32)
+    fed = synth.prompt(cfg, b, steps, 33).astype(np.int32)
+    m.forward(ids, 0)
+    if captured:   # (the captured step of before is not replayed)
+        m.decode_loop(torch.from_numpy(fed[:, 0].copy()).cuda(), n, 4)
+        m.clear_kv_cache()
+        m.forward(ids, 0)
+    _lib.call("rb_selftest_refuse_step", m._m)
+    oracle = util.build_oracle(cfg, w)
+    oracle.forward(torch.from_numpy(ids.astype(np.int64)), 0)
+    for t in range(steps):
+        before = cuda.launch_count()
+        got = m.forward(fed[:, t:t + 1], n + t).reshape(b, -1).float().cpu()
+        assert cuda.launch_count() - before > 6
+        want = oracle.forward(torch.from_numpy(fed[:, t:t + 1].astype(np.int64)), n + t).reshape(b, -1)
+        assert util.logit_error(got, want) <= 2e-2, t
+    again = m.decode_loop(torch.from_numpy(fed[:, 0].copy()).cuda(), n + steps, 6)
+    m.device.synchronize()
+    assert again.shape == (6, b)
+    with pytest.raises(_lib.RaiB200Error):
+        _lib.call("rb_selftest_refuse_step", m._m)   # the plan is gone
+    m.close()

@@ -277,11 +277,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
   if (warp == kWorkWarps) {
     if (lane == 0) {
       const uint64_t policy = ptx::policy_evict_first();
-      // (A slot that was given back without having been waited for must not be armed again: its barrier may still expect what was asked for.
-      // Whoever gives it back so has seen the flag, and who acquires it sees it, too.)
-      auto acquire = [&]() {
-        return ok = ptx::mbar_wait(&sh.empty[r.slot], r.parity ^ 1u, abort_flag, p.wait_cycles) && *abort_flag == 0;
-      };
+      auto acquire = [&]() { return ok = ptx::mbar_wait(&sh.empty[r.slot], r.parity ^ 1u, abort_flag, p.wait_cycles); };
 #pragma unroll 1
       for (int l = 0; l <= p.layers && ok; ++l) {
 #pragma unroll 1
@@ -385,7 +381,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
 #pragma unroll 1
               for (int k = 0; k < stages; ++k) {
                 if ((r.slot & 1) == turn && ok) {
-                  ok = ptx::mbar_wait(&sh.empty[r.slot], r.parity ^ 1u, abort_flag, p.wait_cycles) && *abort_flag == 0;   // (as above)
+                  ok = ptx::mbar_wait(&sh.empty[r.slot], r.parity ^ 1u, abort_flag, p.wait_cycles);
                   uint64_t* bar = &sh.full[r.slot];
                   if (ok) {
                     ptx::mbar_expect_tx(bar, bytes);
@@ -423,13 +419,14 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
     // (A parity tells a slot's use from the one before it, not from the one before that: who does not read every slot in turn first sees that
     // the slot has been left by its last user.  The use before that one has been: copies go round in order, and either this warp has had
     // the slot eight places before this one, or all warps have met since.)
+    // What has not come (somebody gave up) is not given back: its barrier still expects a copy, and nobody may arm it again.
     auto wait_slot = [&](const Ring& at) {
-      ptx::mbar_wait(&sh.empty[at.slot], at.parity ^ 1u, abort_flag, p.wait_cycles);
-      ptx::mbar_wait(&sh.full[at.slot], at.parity, abort_flag, p.wait_cycles);
+      return ptx::mbar_wait(&sh.empty[at.slot], at.parity ^ 1u, abort_flag, p.wait_cycles) &&
+             ptx::mbar_wait(&sh.full[at.slot], at.parity, abort_flag, p.wait_cycles);
     };
-    auto leave_slot = [&](const Ring& at, int n) {
-      __syncwarp();
-      if (lane == 0) release_slot(&sh.empty[at.slot], n);
+    auto leave_slot = [&](const Ring& at, int n, bool came) {
+      came = __all_sync(0xffffffffu, came);
+      if (lane == 0 && came) release_slot(&sh.empty[at.slot], n);
     };
     // acc += W . X^T over the slots of one pass.  A slot belongs to one warp, which takes all its rows: a byte of it is read once from
     // shared memory, and eight slots are at work at a time.  (With a slot's rows shared out among the warps each of them waited for
@@ -450,9 +447,10 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
       Ring mine = r;
       mine.pass(warp, slots);
       if (at >= stages) at -= stages;
+      const bool whole_ring = *abort_flag == 0;   // (no slot that only some warps of an attention gave back: four more would be too many)
 #pragma unroll 1
       for (int turn = warp; turn < stages; turn += kWorkWarps) {
-        wait_slot(mine);
+        const bool came = wait_slot(mine) && whole_ring;
         const int n = min(slices, whole - at * slices);
         const uint32_t base = ring_a + (uint32_t)(mine.slot * slot_bytes);
 #pragma unroll T == 2 ? 2 : 1
@@ -480,7 +478,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
               for (int t = 0; t < T; ++t) mma16816(acc[h * T + t], w[h * T + t], x[2 * (h0 + h)], x[2 * (h0 + h) + 1]);
           }
         }
-        leave_slot(mine, kReleases);
+        leave_slot(mine, kReleases, came);
         mine.slot += kWorkWarps;
         if (mine.slot >= slots) { mine.slot -= slots; mine.parity ^= 1u; }   // (there are at least as many slots as warps)
         at += kWorkWarps;
@@ -637,7 +635,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
           const int at_k = r.slot * slot_bytes;
           const int first = (first_tile + i) * C::kKeys + kw0;
           const bool has_new = newest && i == n - 1, active = first < len;
-          wait_slot(r);
+          bool came = wait_slot(r);
           if (has_new) patch(0, at_k);
           float s[2][4] = {};
           uint32_t pa[4] = {};
@@ -666,7 +664,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
               for (int e = 0; e < 4; ++e) s[nt][e] += odd[nt][e];
           }
           if (has_new) ptx::fence_proxy_async();
-          leave_slot(r, kReleases / C::kWarpsPerTile);
+          leave_slot(r, kReleases / C::kWarpsPerTile, came);
           r.pass(slots);
           if (active) {
             float mx[2] = {-INFINITY, -INFINITY};
@@ -703,7 +701,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
               for (int j = 0; j < D / 8; ++j) { o[j][0] *= corr[0]; o[j][1] *= corr[0]; o[j][2] *= corr[1]; o[j][3] *= corr[1]; }
             }
           }
-          wait_slot(r);
+          came = wait_slot(r);
           const int at_v = r.slot * slot_bytes;
           if (has_new) patch(1, at_v);
           if (active) {
@@ -717,7 +715,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
             }
           }
           if (has_new) ptx::fence_proxy_async();
-          leave_slot(r, kReleases / C::kWarpsPerTile);
+          leave_slot(r, kReleases / C::kWarpsPerTile, came);
           r.pass(slots);
         }
         // ---- the warps' parts of the piece: one scale, then one sum per element in the order of the warps

@@ -78,6 +78,7 @@ struct StepParams {
   size_t layer_stride;                       // elements of one layer's pages
   bool want_head;
   float eps, scale_log2;
+  float squares_of, squares_over;            // what a column is multiplied by before it is squared, and the sum divided by
   bf16 *h, *hw, *attn, *inner, *logits;
   float *qkv_out, *squares, *part_o, *part_ml;
   bf16 *cache_k, *cache_v;
@@ -499,11 +500,15 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
       for (int i = 0; i < kShares; ++i) s += part[i];
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if ((tid & 15) == 0 && (tid >> 4) < m_rows) sh.rstd[tid >> 4] = 1.0f / sqrtf(s / (float)p.hidden + p.eps);
+      if ((tid & 15) == 0 && (tid >> 4) < m_rows) sh.rstd[tid >> 4] = 1.0f / sqrtf(s / p.squares_over + p.eps);
     };
     // what the next norm needs of a finished column of the stream: times its weight, and the square
     auto publish = [&](int c, float v, float gain) {
       p.hw[(size_t)row_e * p.hidden + own0 + c] = __float2bfloat16_rn(v * (p.norm == RB_NORM_RMS_ONE_PLUS ? gain + 1.0f : gain));
+    };
+    auto square = [&](float v) {   // (as the norm's own kernel takes it: RMS divides by the root of the width first, and a mean is in range where a sum is not)
+      v *= p.squares_of;
+      return v * v;
     };
     auto publish_squares = [&](float s) {   // of this thread's columns
       s = warp_sum(s);
@@ -868,7 +873,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
       for (int c = col_e; row_ok && c < own_n; c += 32) {
         const float v = __bfloat162float(p.h[(size_t)row_e * p.hidden + own0 + c]);
         own[row_e * own_rows + c] = v;
-        if (serial) { publish(c, v, __bfloat162float(p.layer[0].norm1_w[own0 + c])); squares += v * v; }
+        if (serial) { publish(c, v, __bfloat162float(p.layer[0].norm1_w[own0 + c])); squares += square(v); }
       }
       if (serial) { publish_squares(squares); arrive(); }
     }
@@ -975,7 +980,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
               float& mine = own[row_e * own_rows + c];
               v = round_bf16((serial ? v : v + e) + mine);
               mine = v;
-              if (serial) { publish(c, v, e); squares += v * v; }
+              if (serial) { publish(c, v, e); squares += square(v); }
               if (!serial || (last && op == kDown)) p.h[(size_t)row_e * p.hidden + y + c] = __float2bfloat16_rn(v);
               continue;
             }
@@ -1075,6 +1080,8 @@ int step_reserve(rb_model* m) {
   p.layers = c.num_hidden_layers; p.hidden = H; p.inter = I; p.nqkv = m->nqkv_l; p.vocab = m->vocab_l;
   p.q_heads = m->nq_l; p.kv_heads = m->nkv_l; p.group = group; p.rot = c.rotary_dim; p.act = c.hidden_act; p.eps = (float)c.norm_eps;
   p.norm = phi2 ? RB_NORM_LAYER : c.arch == RB_ARCH_GEMMA ? RB_NORM_RMS_ONE_PLUS : RB_NORM_RMS;
+  p.squares_of = p.norm == RB_NORM_RMS ? 1.0f / sqrtf((float)H) : 1.0f;
+  p.squares_over = p.norm == RB_NORM_RMS ? 1.0f : (float)H;
   const int64_t n[5] = {p.nqkv, H, I, H, p.vocab}, k[5] = {H, K, H, I, H};
   int most = kPageTokens * ((d + 63) / 64) * 128;
   for (int op = 0; op < 5; ++op) {

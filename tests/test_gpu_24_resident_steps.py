@@ -160,3 +160,23 @@ def test_a_refused_launch_falls_back_to_the_kernels_of_other_steps(cuda, capture
     with pytest.raises(_lib.RaiB200Error):
         _lib.call("rb_selftest_refuse_step", m._m)   # the plan is gone
     m.close()
+
+
+@pytest.mark.parametrize("family", ["qwen2-128", "phi3-96"])
+def test_rows_whose_squares_sum_past_float32(cuda, family):
+    """RMSNorm divides by the root of the width before it squares (rai-nn/src/rms_norm.rs:18-22): a root mean square of 2^60 is in range, the
+    sum of its squares is not.  What layers add to such a stream is nothing, so the logits are those of the embedding's norm."""
+    cfg = _config(family)
+    w = synth.weights(cfg, 35)
+    embed = np.asarray(w["model.embed_tokens.weight"], np.float64)
+    w["model.embed_tokens.weight"] = (embed * 2.0 ** 60 / np.sqrt((embed ** 2).mean())).astype(np.float32)
+    m = Model(cfg, _lib.BF16, cuda, 3, 64, 3)
+    m.update_params(w)
+    ids = np.array([[5], [77], [1030]], np.int32)
+    got = m.forward(ids, 0).reshape(3, -1).float().cpu()
+    rows = torch.from_numpy(embed[ids[:, 0]])
+    rows = rows / (rows ** 2).mean(-1, keepdim=True).sqrt() * torch.from_numpy(np.asarray(w["model.norm.weight"], np.float64))
+    want = rows @ torch.from_numpy(np.asarray(w["lm_head.weight"], np.float64)).T
+    for i in range(3):
+        assert util.logit_error(got[i], want[i]) <= 2e-2, i
+    m.close()

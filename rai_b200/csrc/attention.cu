@@ -229,14 +229,18 @@ attention_kernel(const AParams p, const __grid_constant__ CUtensorMap tm_k, cons
         const int y = (page * p.kv_heads + kvh) * kTile;  // first row of this (page, KV head) in the layer
         uint8_t* ks = kv_s + stage * C::kStageBytes;
         uint8_t* vs = ks + C::kVOffset;
-        // a step reads a tile once: L2 keeps what its kernels share (64 x 2048 keys of qwen2-7b 4.43 -> 4.34 ms a step, 32 x 700 of phi2,
-        // 8 layers, 1018 -> 981 us)
-        const uint64_t policy = ptx::policy_evict_first();
+        // A step reads a tile once: L2 keeps what its kernels share (64 x 2048 keys of qwen2-7b 4.43 -> 4.34 ms a step, 32 x 700 of phi2,
+        // 8 layers, 1018 -> 981 us).  A prompt reads it once per query head of the group and 64 rows, from L2 where it can.
+        [[maybe_unused]] const uint64_t policy = DECODE ? ptx::policy_evict_first() : 0;
+        auto copy = [&](uint8_t* to, const CUtensorMap* map, int x) {
+          if constexpr (DECODE) ptx::tma_load_2d_hint(to, map, &full_bar[stage], x, y, policy);
+          else ptx::tma_load_2d(to, map, &full_bar[stage], x, y);
+        };
         ptx::mbar_expect_tx(&full_bar[stage], C::kStageBytes);
 #pragma unroll
         for (int cb = 0; cb < C::kBlocks; ++cb) {
-          ptx::tma_load_2d_hint(ks + cb * (kTile * 128), &tm_k, &full_bar[stage], cb * 64, y, policy);
-          if (!SHARED) ptx::tma_load_2d_hint(vs + cb * (kTile * 128), &tm_v, &full_bar[stage], cb * 64, y, policy);
+          copy(ks + cb * (kTile * 128), &tm_k, cb * 64);
+          if (!SHARED) copy(vs + cb * (kTile * 128), &tm_v, cb * 64);
         }
       }
       return;

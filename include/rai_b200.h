@@ -801,7 +801,8 @@ int64_t rb_launch_count(rb_ctx* ctx);
  * sites): between rb_profile_start and rb_profile_read every kernel launch of the library is
  * bracketed by CUDA events on the context's stream.  rb_profile_read synchronises, stops profiling
  * and fills out4 = {launches, total milliseconds, algorithmic bytes, floating-point operations} for
- * one kernel class (RB_PROF_*). */
+ * one kernel class (RB_PROF_*).  A single-token step that otherwise runs as one kernel runs as separate launches
+ * meanwhile, so that its classes can be told apart. */
 enum { RB_PROF_GEMM = 0, RB_PROF_ATTENTION = 1, RB_PROF_NORM = 2, RB_PROF_ROPE_KV = 3, RB_PROF_EMBED = 4,
        RB_PROF_ARGMAX = 5, RB_PROF_OTHER = 6, RB_PROF_RECURRENCE = 7, RB_PROF_EXPERTS = 8, RB_PROF_CLASSES = 9 };
 int32_t rb_profile_start(rb_ctx* ctx);

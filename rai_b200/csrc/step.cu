@@ -1144,8 +1144,9 @@ int step_reserve(rb_model* m) {
 // 4 x 2048 704 -> 627 (0.44), 8 x 200 603 -> 537 (0.09), 8 x 2048 813 -> 828 (0.89); phi2 1 x 64 515 -> 384, 8 x 512 577 -> 521 (0.27),
 // 8 x 1500 672 -> 670 (0.78); qwen2-7b 1 x 128 959 -> 910, 8 x 2048 1063 -> 1039 (0.07).  With sixteen sequences (two eights per product)
 // every one of these was slower: phi3-mini 16 x 200 675 -> 706, qwen2-7b 16 x 2048 1086 -> 1164.
+// (Under a per-launch profile the steps are launches of their own: a launch belongs to one class there.)
 bool step_takes(const rb_model* m, int batch) {
-  if (!m->step_plan || batch > kRows || (size_t)batch * m->nqkv_l > m->scratch_floats) return false;
+  if (!m->step_plan || m->ctx->profiling || batch > kRows || (size_t)batch * m->nqkv_l > m->scratch_floats) return false;
   double tokens = 0;
   for (int b = 0; b < batch; ++b) tokens += m->cache->host_lens[b];
   return tokens * m->step_plan->token_bytes <= 0.75 * m->step_plan->layer_bytes;
@@ -1179,13 +1180,6 @@ int step_forward(rb_model* m, int batch, bool want_head, bool* ran) {
   const void* x[5] = {p.hw, p.attn, p.hw, p.inner, p.hw};
   const int k[5] = {H, K, H, I, H};
   for (int op = 0; op < 5; ++op) RB_TRY(tmap_slices_bf16(x[op], batch, k[op], batch, p.share[op].slices, &p.x[op]));
-  const double layer = (double)p.nqkv * H + (double)H * K + (c.arch == RB_ARCH_PHI2 ? 2.0 : 3.0) * I * H, head = want_head ? (double)p.vocab * H : 0.0;
-  double bytes = 2.0 * (p.layers * layer + head), flops = 2.0 * batch * (p.layers * layer + head);
-  for (int b = 0; b < batch; ++b) {
-    bytes += 4.0 * p.layers * m->cache->host_lens[b] * p.kv_heads * m->d;
-    flops += 4.0 * p.layers * m->cache->host_lens[b] * p.q_heads * m->d;
-  }
-  ProfScope prof(ctx, RB_PROF_GEMM, bytes, flops);
   cudaError_t e = cudaErrorCooperativeLaunchTooLarge;
   if (!m->step_plan->refused) {
     switch (m->d) {

@@ -180,3 +180,28 @@ def test_rows_whose_squares_sum_past_float32(cuda, family):
     for i in range(3):
         assert util.logit_error(got[i], want[i]) <= 2e-2, i
     m.close()
+
+
+@pytest.mark.parametrize("family", ["phi3-96", "phi2-80"])
+def test_a_profile_of_a_step_tells_its_classes_apart(cuda, family):
+    """A launch belongs to one class of the per-launch profile, so a step under it runs as launches of its own; the next one does not."""
+    cfg = _config(family)
+    b, n = 2, 70
+    m = Model(cfg, _lib.BF16, cuda, b, 128, b * n)
+    m.update_params(synth.weights(cfg, 37))
+    m.forward(synth.prompt(cfg, b, n, 38).astype(np.int32), 0)
+    token = np.ones((b, 1), np.int32)
+    _lib.call("rb_profile_start", cuda.ctx)
+    m.forward(token, n)
+    out, seen = (ctypes.c_double * 4)(), {}
+    for i, name in enumerate(("gemm", "attention", "norm")):
+        _lib.call("rb_profile_read", cuda.ctx, i, out)
+        seen[name] = list(out)
+    layers, kv = cfg["num_hidden_layers"], cfg["num_key_value_heads"]
+    keys_values = 2 * 2 * b * (n + 1) * kv * configs.head_dim(cfg)
+    assert seen["attention"][0] == layers and seen["attention"][2] >= layers * keys_values, seen
+    assert seen["norm"][0] > layers and seen["gemm"][0] > 3 * layers, seen
+    before = cuda.launch_count()
+    m.forward(token, n + 1)
+    assert cuda.launch_count() - before <= 6
+    m.close()

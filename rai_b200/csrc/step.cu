@@ -565,6 +565,9 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
       const int grp = warp / C::kWarpsPerTile, kw0 = (warp % C::kWarpsPerTile) * 16;
       const int g = lane >> 2, t4 = lane & 3;
       const int half = p.rot >> 1;
+      // Whoever gave up has no row to append: what it would write (not a number, maybe) lies behind the cached length, where it is masked out of
+      // later prompts' products as zero times that.
+      const bool sound = *abort_flag == 0;
       while (w.left > 0) {
         int first_tile;
         const int n = piece_of(w, first_tile), b = w.b, kvh = w.kvh, head = kvh * p.group, len = sh.len[b], pos = len - 1;
@@ -580,7 +583,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
             if (r < p.group) { store8(reinterpret_cast<bf16*>(q_s + r * C::kQRow) + at, v); return; }
             bf16* keep = new_kv + (r - p.group) * D + at;
             store8(keep, v);
-            *reinterpret_cast<uint4*>((r == p.group ? p.cache_k : p.cache_v) + new_row + at) = *reinterpret_cast<const uint4*>(keep);
+            if (sound) *reinterpret_cast<uint4*>((r == p.group ? p.cache_k : p.cache_v) + new_row + at) = *reinterpret_cast<const uint4*>(keep);
           };
 #pragma unroll 1
           for (int it = tid; it < total; it += 256) {

@@ -205,3 +205,26 @@ def test_a_profile_of_a_step_tells_its_classes_apart(cuda, family):
     m.forward(token, n + 1)
     assert cuda.launch_count() - before <= 6
     m.close()
+
+
+@pytest.mark.parametrize("family", ["qwen2-128", "phi2-80"])
+def test_a_step_that_gives_up_leaves_the_cache_alone(cuda, family):
+    """No barrier opens, so no block has a key or value to append: the rows behind the cached ones stay as they are, zero in a new cache.  (Rows that are
+    not numbers there would reach later sequences of the same pages, whose masked probabilities are zero times them.)"""
+    cfg = _config(family)
+    b, n = 3, 200
+    m = Model(cfg, _lib.BF16, cuda, b, 256, b * n)
+    m.update_params(synth.weights(cfg, 43))
+    m.forward(synth.prompt(cfg, b, n, 44).astype(np.int32), 0)
+    _lib.call("rb_set_wait_budget_us", cuda.ctx, 500)
+    try:
+        _lib.call("rb_selftest_spoil_step", m._m)
+        with pytest.raises(_lib.RaiB200Error, match="0x57e9"):
+            m.forward(np.array([[1], [2], [3]], np.int32), n)
+    finally:
+        _lib.call("rb_set_wait_budget_us", cuda.ctx, 1000000)
+    for layer in range(cfg["num_hidden_layers"]):
+        for seq in range(b):
+            for head in range(cfg["num_key_value_heads"]):
+                assert not any((x != 0).any() for x in m.kv_read(layer, seq, head, n, 1)), (layer, seq, head)
+    m.close()

@@ -32,13 +32,17 @@ inline SplitCost joint_split_cost(int tile_bytes, int sums, int sm_count) {
 // One block per pair keeps its copies coming and hands nothing over; splitting pays where pairs are few and their tiles take longer
 // than the hand-over.  Blocks run in rounds of `slots`; each round that splitting adds costs a start.  Gains below 1 % are left alone:
 // of many pairs they are no more than the end of the last round, which is not as even as this.
+inline double key_split_cost(const SplitCost& c, int pairs, int tiles, int s) {
+  const int rounds = (pairs * s + c.slots - 1) / c.slots;
+  double cost = rounds * (c.start + c.tile * ((tiles + s - 1) / s));
+  if (s > 1) cost += (c.hand + c.part * s) * std::max(1.0, (double)pairs / c.slots);
+  return cost;
+}
 inline int pick_key_splits(const SplitCost& c, int pairs, int tiles) {
   int best = 1;
   double best_cost = 1e30;
   for (int s = 1; s <= std::min(tiles, 32); ++s) {
-    const int rounds = (pairs * s + c.slots - 1) / c.slots;
-    double cost = rounds * (c.start + c.tile * ((tiles + s - 1) / s));
-    if (s > 1) cost += (c.hand + c.part * s) * std::max(1.0, (double)pairs / c.slots);
+    const double cost = key_split_cost(c, pairs, tiles, s);
     if (cost < best_cost) {
       best_cost = s == 1 ? 0.99 * cost : cost;
       best = s;

@@ -36,6 +36,7 @@
 #include "model.h"
 #include "ptx.cuh"
 #include "step.h"
+#include "step_rule.h"
 
 namespace rb {
 
@@ -206,8 +207,9 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(const __grid_constant
   }
   __syncthreads();
 
-  // ---- how the keys are shared out: all pairs (sequence, KV head) in pieces of at most `most / (lane + 1)` tiles, in a line, the same number
-  // of pieces for every CTA.  The cheapest of 16 ways, in units of 0.1 us: a tile 4, a piece 35 (rows in, parts out), cut pairs 25.
+  // ---- how the keys are shared out (step_pieces of step_rule.h does the same on the host): all pairs (sequence, KV head) in pieces of at
+  // most `most / (lane + 1)` tiles, in a line, the same number of pieces for every CTA.  The cheapest of 16 ways, in units of 0.1 us: a
+  // tile 4, a piece 35 (rows in, parts out), cut pairs 25.
   if (warp == 0) {
     int most = 0;
     for (int b = 0; b < m_rows; ++b) most = max(most, sh.tiles[b]);
@@ -1142,17 +1144,22 @@ int step_reserve(rb_model* m) {
   return RB_OK;
 }
 
-// Up to eight sequences, and no more cached bytes than three quarters of the weights': the attention phase reads K and V at 5 TB/s, a launch
-// of its own at 5.5.  us per step of 8 layers, as launches -> here (K and V without the L2 hint on both sides), and cached bytes to weights: phi3-mini 1 x 2048 keys 619 -> 516 (0.11),
-// 4 x 2048 704 -> 627 (0.44), 8 x 200 603 -> 537 (0.09), 8 x 2048 813 -> 828 (0.89); phi2 1 x 64 515 -> 384, 8 x 512 577 -> 521 (0.27),
-// 8 x 1500 672 -> 670 (0.78); qwen2-7b 1 x 128 959 -> 910, 8 x 2048 1063 -> 1039 (0.07).  With sixteen sequences (two eights per product)
+// Up to eight sequences, no more cached bytes than three quarters of the weights' (a step of more streams as fast in launches of its own), and an
+// attention phase that is not longer than the launches' by more than those lose between kernels (step_rule.h).  us per step of 8 layers, as launches -> here,
+// and cached bytes to weights: phi3-mini 1 x 3500 keys 597 -> 507 (0.19), 4 x 2048 662 -> 574 (0.44), 8 x 200 566 -> 503 (0.09), 8 x 1700 721 -> 705 (0.74); phi2
+// 1 x 17 473 -> 349, 8 x 512 528 -> 470 (0.27), 8 x 1400 608 -> 594 (0.73); qwen2-7b 1 x 17 782 -> 743, 8 x 4500 928 -> 903 (0.16); layers of 97 MB,
+// 1 x 100 and 8 x 500 keys: qwen2 400 -> 294 and 455 -> 336, phi3 374 -> 289 and 431 -> 390.  With sixteen sequences (two eights per product)
 // every one of these was slower: phi3-mini 16 x 200 675 -> 706, qwen2-7b 16 x 2048 1086 -> 1164.
 // (Under a per-launch profile the steps are launches of their own: a launch belongs to one class there.)
 bool step_takes(const rb_model* m, int batch) {
-  if (!m->step_plan || m->ctx->profiling || batch > kRows || (size_t)batch * m->nqkv_l > m->scratch_floats) return false;
+  const StepPlan* plan = m->step_plan;
+  if (!plan || m->ctx->profiling || batch > kRows || (size_t)batch * m->nqkv_l > m->scratch_floats) return false;
+  const int32_t* lens = m->cache->host_lens.data();
   double tokens = 0;
-  for (int b = 0; b < batch; ++b) tokens += m->cache->host_lens[b];
-  return tokens * m->step_plan->token_bytes <= 0.75 * m->step_plan->layer_bytes;
+  for (int b = 0; b < batch; ++b) tokens += lens[b];
+  const StepParams& p = plan->p;
+  return tokens * plan->token_bytes <= 0.75 * plan->layer_bytes &&
+         step_attention_pays(lens, batch, p.kv_heads, p.group, m->d, m->ctx->sm_count, p.most_pieces);
 }
 
 int step_spoil(rb_model* m) {

@@ -228,3 +228,17 @@ def test_a_step_that_gives_up_leaves_the_cache_alone(cuda, family):
             for head in range(cfg["num_key_value_heads"]):
                 assert not any((x != 0).any() for x in m.kv_read(layer, seq, head, n, 1)), (layer, seq, head)
     m.close()
+
+
+@pytest.mark.parametrize("batch,one", [(6, True), (7, False)])
+def test_pairs_that_leave_blocks_idle_stay_on_launches(cuda, batch, one):
+    """24 heads: 6 sequences are 144 pairs for 148 blocks, 7 are 168 (84 blocks would walk two pairs each, as long as 84 blocks alone can)."""
+    cfg = _config("phi3-96")
+    cfg["max_position_embeddings"] = 2048
+    m = Model(cfg, _lib.BF16, cuda, batch, 1664, batch)
+    m.update_params(synth.weights(cfg, 45))
+    _lib.call("rb_kv_cache_set_len", _lib.lib().rb_model_kv_cache(m._m), batch, 1590)
+    before = cuda.launch_count()
+    m.forward(np.ones((batch, 1), np.int32), 1590)
+    assert (cuda.launch_count() - before <= 6) == one
+    m.close()

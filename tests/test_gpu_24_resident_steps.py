@@ -242,3 +242,26 @@ def test_pairs_that_leave_blocks_idle_stay_on_launches(cuda, batch, one):
     m.forward(np.ones((batch, 1), np.int32), 1590)
     assert (cuda.launch_count() - before <= 6) == one
     m.close()
+
+
+@pytest.mark.parametrize("family", ["qwen2-128", "phi2-80"])
+@pytest.mark.parametrize("batch", [1, 8])
+def test_a_vocabulary_that_takes_several_passes(cuda, family, batch):
+    """40007 rows are three passes of 91 for each of 148 blocks: the last block has none, the one before it two."""
+    cfg = _config(family)
+    cfg["vocab_size"] = 40007
+    w = synth.weights(cfg, 41)
+    n = 65
+    m = Model(cfg, _lib.BF16, cuda, batch, 128, batch * n)
+    m.update_params(w)
+    ids = synth.prompt(cfg, batch, n + 1, 42).astype(np.int32)
+    m.forward(ids[:, :n], 0)
+    before = cuda.launch_count()
+    got = m.forward(ids[:, n:], n).reshape(batch, -1).float().cpu()
+    assert cuda.launch_count() - before <= 6
+    oracle = util.build_oracle(cfg, w)
+    oracle.forward(torch.from_numpy(ids[:, :n].astype(np.int64)), 0)
+    want = oracle.forward(torch.from_numpy(ids[:, n:].astype(np.int64)), n).reshape(batch, -1)
+    for i in range(batch):
+        assert util.logit_error(got[i], want[i]) <= 2e-2, i
+    m.close()

@@ -3,21 +3,23 @@
 //
 // What bounds such a step beside its bytes is the hand-overs between the products, the attention and the norms of a layer: as
 // launches of their own each costs 4 to 8 us from the last store of one to the first product of the next, seven to nine times a
-// layer.  Here one CTA stays on every SM and the phases of a layer follow one another through grid-wide barriers (five a layer, 2 us from the
-// last arrival to the first product), while the copies of weights and cached keys and values, which depend on nothing, run ahead through
+// layer.  Here one CTA stays on every SM and the phases of a layer follow one another through grid-wide barriers (five a layer, about 2 us
+// each by themselves), while the copies of weights and cached keys and values, which depend on nothing, run ahead through
 // all of them: a ring of shared memory (190 KB an SM, 4.5 us of HBM over the GPU) takes the tiles of the next phase while this one
-// waits.  us per step of 8 layers, seven launches a layer -> here: phi2 (157 MB a layer) 1 x 64 keys 515 -> 383, 8 x 512 576 -> 508;
-// phi3-mini (226 MB) 1 x 2048 613 -> 507, 4 x 2048 701 -> 613; qwen2-7b (466 MB) 1 x 128 957 -> 913.  A layer of phi3-mini with 4 x 2048
-// keys takes 69 us, of which 50 are its 326 MB at the copy rate; inside the phases HBM delivers 6 TB/s (5 in attention).
+// waits.  us per step of 8 layers and a vocabulary of 1024, seven launches a layer -> here: phi2 (157 MB a layer) 1 x 17 keys 473 -> 349, 8 x 512
+// 528 -> 470; phi3-mini (226 MB) 1 x 3500 597 -> 507, 4 x 2048 662 -> 574; qwen2-7b (466 MB) 1 x 17 782 -> 743.  A layer of phi3-mini
+// takes 54 us with 17 keys, 35 of them its weights at the copy rate, and 72 with 4 x 2048 keys (50); a further MB of weights costs what HBM
+// takes for it (97 -> 145 MB a layer), a further MB of keys and values 5.6 TB/s (8 x 200 -> 8 x 1600).  DRAM reads are 0.5 to 2.5 % above the bytes.
 //
 //   warp 8      weights, keys and values: TMA tiles into the ring in the order of the program, whatever phase the rest is in
 //   warps 9, 10 wait at the barriers; then the activations that belong to each weight tile (a few KB from L2) into the same slot
 //   warps 0-7   products (mma.sync), attention, epilogues
 //
-// Rows of a weight matrix are shared out evenly over the CTAs (3072 rows are 21 each for 147 of 148), so no product is cut along K over CTAs, no
-// sums travel between SMs and a result does not depend on how many rows the call has.  That is also why the products are mma.sync: a
+// Rows of a weight matrix are shared out evenly over the CTAs (3072 rows are 21 each for 147 of 148), so no product is cut along K over CTAs and no
+// sums travel between SMs.  (In what order the eight warps' sums meet depends on the rows of the call, and into what pieces the attention is
+// cut on all its lengths, so a sequence's last bits may.)  That is also why the products are mma.sync: a
 // tile of 128 rows, which tcgen05 wants, would leave most SMs without work or cut K sixfold, and at eight rows of X the tensor cores
-// have nothing to do anyway.  With more rows the activations' way through L2 costs more than the launches did (see step_takes).
+// have nothing to do anyway (active 7 to 9 % of the time).  With more rows the activations' way through L2 costs more than the launches did (see step_takes).
 //
 // A CTA owns the same few columns of the residual stream all through the step and keeps them in shared memory.  The RMS norms need no
 // phase of their own: whoever finishes a column of the stream also writes it times the next norm's weight, and its square joins a
@@ -166,8 +168,7 @@ struct Shared {
 
 static_assert(sizeof(Shared) <= 3072, "static shared memory");
 
-// Where a CTA begins its way along K.  (All of them at the same place would ask the same few lines of X of L2 at the same time:
-// 26 ns a line, 7B model, 16 rows.)
+// Where a CTA begins its way along K.  (All of them at the same place would ask the same few lines of X of L2 at the same time.)
 __device__ __forceinline__ int first_stage(int cta, int ctas, int stages) { return cta * stages / ctas; }
 __device__ __forceinline__ void release_slot(uint64_t* bar, int n) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(ptx::smem_u32(bar)), "r"(n) : "memory");
@@ -1072,7 +1073,7 @@ int step_reserve(rb_model* m) {
   const int64_t cache_rows = (int64_t)kv->num_pages * kv->kv_heads * kPageTokens;
   const double layer_bytes = 2.0 * ((double)m->nqkv_l * H + (double)H * K + (phi2 ? 2.0 : 3.0) * I * H);
   // Models of up to 96 MB a layer have faster steps as five launches a layer (gemm_rows.cu): 24 layers of 28 MB, one row, 0.66 ms against
-  // 0.69 here.  Heads of 256 (gemma-2b, 8 layers, 8 x 1024 keys: 805 us as launches, 883 here) would want two slots for a tile.
+  // 0.69 here.  (Layers of 97, 110, 125 and 145 MB take 0.72 to 0.93 of the launches' time here, 24 points each; between 28 and 97 nothing was measured.)  Heads of 256 (gemma-2b, 8 layers, 8 x 1024 keys: 805 us as launches, 883 here) would want two slots for a tile.
   if (c.dtype != RB_BF16 || c.tp_size != 1 || layer_bytes <= (double)(96 << 20) || c.num_hidden_layers > kStepLayers || H % 64 || I % 64 ||
       K % 64 || c.hidden_act == RB_ACT_XIELU || group > 16 || !(d == 64 || d == 80 || d == 96 || d == 128) || c.rotary_dim % 16 ||
       c.rotary_dim > d || (d - c.rotary_dim) % 8 || (H + ctas - 1) / ctas > kOwnColumns || cache_rows * c.num_hidden_layers >= (1LL << 31) ||

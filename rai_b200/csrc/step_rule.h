@@ -37,7 +37,8 @@ inline StepPieces step_pieces(const int* lens, int batch, int kv_heads, int ctas
 // Microseconds of both: here the busiest CTA's pieces (3.5 each, 2.5 where pairs are cut, 0.5 a tile, 0.72 where several query heads of 128
 // multiply it), there the account of attention_splits.h, but not below the bytes at 6 TB/s.  us a layer, launches -> one kernel:
 // phi3-mini 5 x 1500 84.7 -> 82.8, 5 x 2000 90.8 -> 91.9, 5 x 2700 99.0 -> 101.6, 8 x 1700 90.1 -> 88.0, 4 x 3400 91.6 -> 84.1; phi2 5 x 1500
-// 75.7 -> 74.0, 5 x 2000 81.3 -> 83.6; qwen2-7b 8 x 16000 142.8 -> 140.7, 8 x 20000 152.1 -> 159.0, 1 x 90000 148.0 -> 155.6.
+// 75.7 -> 74.0, 5 x 2000 81.3 -> 83.6; qwen2-7b 8 x 16000 142.8 -> 140.7, 1 x 90000 148.0 -> 155.6.  Not
+// caught: qwen2-7b 8 x 20000 152.1 -> 159.0 (288 pieces of 35 tiles, two a CTA, run into the bytes' time).
 inline bool step_attention_pays(const int* lens, int batch, int kv_heads, int group, int head_dim, int ctas, int most_pieces) {
   const StepPieces w = step_pieces(lens, batch, kv_heads, ctas, most_pieces);
   const double tile = head_dim > 96 && group > 1 ? 0.72 : 0.5;
